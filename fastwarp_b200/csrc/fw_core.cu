@@ -550,18 +550,42 @@ __global__ void __launch_bounds__(256) k_resample(DevGrid d, DevGrid s, const fl
         out[l + q * ops] = in ? lin_at_index(f + q * fps, s.nx, s.ny, s.nz, c[0], c[1], c[2]) : 0.0f;
 }
 
-// field_ops.rs:191-203: atomic max of |u/sp| as float bits (non-negative; NaN wins).
+// field_ops.rs:191-203: max of |u/sp| as float bits (non-negative; NaN wins). A stream over the
+// three planes, bound by HBM: 16-byte loads (every plane starts on 256 bytes), one resident wave
+// of blocks striding over the field, and one atomic a block. A voxel a thread with an atomic a
+// warp queued 267 K atomics on one address at 193 x 229 x 193: 202 us, 39 us with this grid.
 __global__ void __launch_bounds__(256) k_max_norm(FieldArgs a, const float* __restrict__ u,
                                                   unsigned int* __restrict__ max_bits) {
-    long long l = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    float v = 0.0f;
-    if (l < a.g.n) {
-        float x = u[l] / (float)a.g.sp[0], y = u[l + a.ps] / (float)a.g.sp[1],
-              z = u[l + 2 * a.ps] / (float)a.g.sp[2];
-        v = nan_canon(sqrtf(x * x + y * y + z * z));
+    __shared__ float wm[8];
+    const float sx = (float)a.g.sp[0], sy = (float)a.g.sp[1], sz = (float)a.g.sp[2];
+    float best = 0.0f;
+    auto take = [&](float vx, float vy, float vz) {
+        const float x = vx / sx, y = vy / sy, z = vz / sz;
+        const float v = nan_canon(sqrtf(x * x + y * y + z * z));
+        best = __int_as_float(max(__float_as_int(best), __float_as_int(v)));
+    };
+    const long long n4 = a.g.n / 4, t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    for (long long q = t; q < n4; q += (long long)gridDim.x * blockDim.x) {
+        const float4 vx = __ldg(reinterpret_cast<const float4*>(u) + q);
+        const float4 vy = __ldg(reinterpret_cast<const float4*>(u + a.ps) + q);
+        const float4 vz = __ldg(reinterpret_cast<const float4*>(u + 2 * a.ps) + q);
+        take(vx.x, vy.x, vz.x);
+        take(vx.y, vy.y, vz.y);
+        take(vx.z, vy.z, vz.z);
+        take(vx.w, vy.w, vz.w);
     }
-    v = warp_max_f(v);
-    if ((threadIdx.x & 31) == 0 && v > 0.0f) atomicMax(max_bits, __float_as_uint(v));
+    if (t < a.g.n - 4 * n4) {  // the last one to three voxels
+        const long long l = 4 * n4 + t;
+        take(u[l], u[l + a.ps], u[l + 2 * a.ps]);
+    }
+    best = warp_max_f(best);
+    if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = best;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w)
+            best = __int_as_float(max(__float_as_int(best), __float_as_int(wm[w])));
+        if (best > 0.0f || isnan(best)) atomicMax(max_bits, __float_as_uint(best));
+    }
 }
 
 // Fixed-order last-block reduction: every block writes `k` partials at its index; the last
@@ -753,7 +777,8 @@ int launch_image_product(fw_ctx* ctx, const fw_image* a, const fw_image* b, fw_i
 
 int launch_max_norm(fw_ctx* ctx, const fw_field* f, unsigned int* d_max_bits) {
     FieldArgs a{dev_grid(f->grid), f->ps};
-    k_max_norm<<<blocks_for(a.g.n), 256, 0, ctx->stream>>>(a, f->d, d_max_bits);
+    const unsigned int blocks = std::min(blocks_for((a.g.n + 3) / 4), 8u * (unsigned int)ctx->num_sms);
+    k_max_norm<<<blocks, 256, 0, ctx->stream>>>(a, f->d, d_max_bits);
     return check_launch(ctx, "k_max_norm");
 }
 
