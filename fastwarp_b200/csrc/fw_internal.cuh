@@ -220,15 +220,11 @@ __device__ __forceinline__ void lin_axis(double c, int n, int& b, float& w) {
     w = (d <= 0.0 || b + 1 > n - 1) ? 0.0f : (float)d;
 }
 
-// interp.rs:43-85: LinearInterpolateImageFunction::EvaluateAtContinuousIndex (no bounds check).
+// interp.rs:43-85: LinearInterpolateImageFunction::EvaluateAtContinuousIndex (no bounds check),
+// from the three axes' bases and weights.
 // Voxel offsets are 32-bit (grids hold fewer than 2^31 voxels).
-__device__ __forceinline__ float lin_at_index(const float* __restrict__ img, int nx, int ny,
-                                              int nz, double cx, double cy, double cz) {
-    int bx, by, bz;
-    float wx, wy, wz;
-    lin_axis(cx, nx, bx, wx);
-    lin_axis(cy, ny, by, wy);
-    lin_axis(cz, nz, bz, wz);
+__device__ __forceinline__ float lin_at_axes(const float* __restrict__ img, int nx, int ny, int bx,
+                                             float wx, int by, float wy, int bz, float wz) {
     const unsigned int sy = (unsigned int)nx, sz = (unsigned int)nx * (unsigned int)ny;
     const unsigned int b = (unsigned int)bx + sy * (unsigned int)by + sz * (unsigned int)bz;
     const unsigned int ox = wx > 0.0f ? 1u : 0u;
@@ -248,6 +244,16 @@ __device__ __forceinline__ float lin_at_index(const float* __restrict__ img, int
         return fmaf(y1 - y0, wz, y0);
     }
     return y0;
+}
+
+__device__ __forceinline__ float lin_at_index(const float* __restrict__ img, int nx, int ny,
+                                              int nz, double cx, double cy, double cz) {
+    int bx, by, bz;
+    float wx, wy, wz;
+    lin_axis(cx, nx, bx, wx);
+    lin_axis(cy, ny, by, wy);
+    lin_axis(cz, nz, bz, wz);
+    return lin_at_axes(img, nx, ny, bx, wx, by, wy, bz, wz);
 }
 
 // field_ops.rs:143-172: VectorLinearInterpolateImageFunction (neighbours clamped, weights 1-d, d)
@@ -364,35 +370,6 @@ __device__ __forceinline__ bool axis_probe_inside(const DevGrid& g, int i, int j
     double c[3];
     probe_index(g, i, j, k, d, sign, c);
     return c[d] >= -0.5 && c[d] < (double)n - 0.5;
-}
-
-// interp.rs:96-120 at voxel (x, y, z) from global memory. On an identity-direction grid the
-// probes at +-half a spacing lerp halfway toward the neighbours along the axis (the face voxels
-// decided by the exact probe test); otherwise the exact probes.
-__device__ __forceinline__ void central_difference_voxel(const float* __restrict__ img,
-                                                         const DevGrid& g, bool identity,
-                                                         const double isp[3], int x, int y,
-                                                         int z, float out[3]) {
-    if (!identity) {
-        central_difference_exact(img, g, x, y, z, out);
-        return;
-    }
-    const int nn[3] = {g.nx, g.ny, g.nz};
-    const int pos[3] = {x, y, z};
-    const long long st[3] = {1, (long long)g.nx, (long long)g.nx * g.ny};
-    const long long l = x + st[1] * y + st[2] * z;
-    const float v = __ldg(img + l);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        out[d] = 0.0f;
-        if (!axis_probe_inside(g, x, y, z, d, -1.0, nn[d]) ||
-            !axis_probe_inside(g, x, y, z, d, +1.0, nn[d]))
-            continue;
-        const int p = pos[d];
-        const float v2 = p < nn[d] - 1 ? fmaf(__ldg(img + l + st[d]) - v, 0.5f, v) : v;
-        const float v1 = p > 0 ? fmaf(v - __ldg(img + l - st[d]), 0.5f, __ldg(img + l - st[d])) : v;
-        out[d] = (float)((double)(v2 - v1) * isp[d]);
-    }
 }
 
 // Thread mapping of the gather sweeps (warp, compose): a block of 256 threads is a 32 x 8 tile of
@@ -623,7 +600,7 @@ namespace fw {
 // sequence of kernels without host read-back (capturable in a graph): the two derivative fields,
 // and at `publish` on the device [value (fixed, moving), |d_fixed|^2, |d_moving|^2, 0,
 // value (moving, fixed), status] (status as dense_mi_status reads it).
-int dense_mi_create(fw_ctx* ctx, int bins, long long n, fw_dense_mi** out);
+int dense_mi_create(fw_ctx* ctx, int bins, const HostGrid& g, fw_dense_mi** out);
 void dense_mi_free(fw_dense_mi* d);
 int enqueue_dense_mi_pair(fw_ctx* ctx, const fw_image* f, const fw_image* m, const fw_image* fm,
                           const fw_image* mm, fw_field* d_fixed, fw_field* d_moving,

@@ -144,7 +144,7 @@ int alloc_level_work(fw_ctx* ctx, const fw_syn_recipe* r, Level& L) {
     if (L.fmask && L.mmask) FW_TRY(new_image(ctx, L.grid, &L.valid));
     bool mattes = false;
     for (int c = 0; c < L.channels; ++c) mattes = mattes || r->channel_metrics[c] == FW_METRIC_MATTES;
-    if (mattes) FW_TRY(dense_mi_create(ctx, r->mi_bins, L.grid.count(), &L.mi));
+    if (mattes) FW_TRY(dense_mi_create(ctx, r->mi_bins, L.grid, &L.mi));
     return 0;
 }
 
@@ -611,7 +611,7 @@ int kernels_per_iteration(const fw_syn_recipe* r, int mask_warps) {
             (r->total_field_variance > 0.0 ? 4 : 0) + 1 /*inversion inits*/ + 1 /*record*/ +
             mask_warps + (mask_warps == 2 ? 1 : 0) /*product*/;
     for (int c = 0; c < r->channels; ++c)
-        if (r->channel_metrics[c] == FW_METRIC_MATTES) k += 6;  // 7 dense MI kernels, not 1 CC
+        if (r->channel_metrics[c] == FW_METRIC_MATTES) k += 3;  // 4 dense MI kernels, not 1 CC
     return k;
 }
 

@@ -125,6 +125,45 @@ def test_sampled_mi_at_the_config2_finest_level_matches_the_oracle(backend):
     assert own.num_valid() == level.num_valid()
 
 
+@pytest.mark.parametrize("scale,shift", [(0.8, 0.0), (1.0, 3.25), (1.4, -2.5)])
+def test_terms_away_from_their_clamped_bin_follow_the_definition(backend, scale, shift):
+    """A binning whose bin size does not belong to its range: terms beyond the clamped bins' [0, 1],
+    where the spline's pieces (and its zero) come from its definition."""
+    og, g, f, m, kept, fbin, b = setup(seed=31)
+    b.moving_bin_size *= scale
+    b.moving_normalized_min = b.moving_min / b.moving_bin_size - 2.0 + shift
+    level = CudaLinearEngine(backend).prepare_level(g, m, kept, fbin, b)
+    kw = transforms(tuple(kept.mean(0)))["euler"]
+    v, d = level.value_and_derivative(linear_transform(**kw))
+    wv, wd, wn, _ = O.mi_evaluate(b, og, m, kept, fbin, O.linear_transform(**kw))
+    # float32 interpolation (6e-8 of a bin's slope) and the 2^-32 fixed point: the file's bounds
+    assert abs(v - wv) <= 1e-5 * abs(wv)
+    assert np.linalg.norm(d - wd) <= 5e-4 * np.linalg.norm(wd)
+    assert level.num_valid() == wn
+
+
+def test_dense_histogram_merges_its_words_before_they_overflow(backend):
+    """110 M voxels, most of them in one cell: more addends a block than a 32-bit word of the
+    block's histogram takes, so blocks merge twice. The image repeats a slab ten times, whose
+    joint PDF (and MI) it shares."""
+    rng = np.random.default_rng(3)
+    slab = np.where(rng.random((48, 480, 481)) < 0.02, rng.random((48, 480, 481)), 0.25)
+    f = slab.astype(np.float32)
+    m = np.where(f == 0.25, np.float32(0.5), f * f).astype(np.float32)
+    out = []
+    for reps in (1, 10):
+        g = make_grid((481, 480, 48 * reps))
+        fi = backend.upload_image(g, np.tile(f, (reps, 1, 1)))
+        mi = backend.upload_image(g, np.tile(m, (reps, 1, 1)))
+        (v0, d0), (v1, d1) = backend.mi_value_derivative_pair(fi, mi, 32)
+        out.append((v0, v1))
+        for b in (fi, mi, d0, d1):
+            b.free()
+    backend.release_idle_buffers()
+    # exact integer histograms, ten times one another: only the f64 logarithms' rounding is left
+    assert np.allclose(out[0], out[1], rtol=1e-12, atol=0.0)
+
+
 def test_all_samples_outside_is_an_error(backend):
     from fastwarp_b200 import FastwarpError
     og, g, f, m, kept, fbin, b = setup()
