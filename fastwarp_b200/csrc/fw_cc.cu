@@ -8,12 +8,21 @@
 // Kernel design (sm_100a): one CTA owns a TX x TY column tile and marches along z over a chunk
 // of slices. The z window comes first, as running sums over the tile's halo columns kept in
 // shared memory (entering slice added, leaving slice subtracted); the y and x box passes then run
-// on those sums. Sums are float64: products of float32 voxels are exact in float64, so the
-// centred second moments (sum f^2 - (sum f)^2 / n) keep their precision in flat bright regions
-// where float32 cancels. The window planes never touch HBM: the kernel reads the two images (the
-// leaving slice and the halo a second time, from L2) and writes the two derivative fields. Shared
-// memory holds the z sums, the y sums and a few raw slices (58 KB at r = 4), and 80 registers a
-// thread let three CTAs share an SM and hide each other's float64 and load latency.
+// on those sums, eight outputs an item by suffix and prefix sums (window_sums). Sums are float64:
+// products of float32 voxels are exact in float64, so the centred second moments
+// (sum f^2 - (sum f)^2 / n) keep their precision in flat bright regions where float32 cancels. The
+// window planes never touch HBM: the kernel reads the two images (the leaving slice and the halo a
+// second time, from L2) and writes the two derivative fields.
+//
+// What bounds it: shared memory (two thirds of its bandwidth) and issue (60 %), at three CTAs of 8
+// warps an SM (80 registers a thread, 60 KB of shared memory); the float64 pipe is a fifth busy.
+// The pair's whole call at 193 x 229 x 193, r = 4: 400 us with 64 additions an x group and 20 a y
+// group, window counters, and the face tests and float64 scaling of the gradients at every voxel;
+// 325 us now. Masked, r = 3, 181 x 217 x 165 on a rotated grid with every probe from global memory in
+// float64: 458 us; 328 us with the probes' common corners and weights on the raw slices.
+// Measured and dropped: z sums in registers (spills at three CTAs: 521 us), 16 rows a tile with one
+// or two voxels a thread (363-424 us), two CTAs an SM without spills (374 us), thinner z chunks on
+// coarse grids (no change: the call's fixed cost).
 #include <cuda_runtime.h>
 
 #include <cfloat>
@@ -27,40 +36,53 @@ namespace fw {
 namespace {
 
 constexpr int TX = 32;
+constexpr int CC_TY = 8;         // rows of a tile
+constexpr int CC_NT = 256;       // threads of a CTA
+
+// Kinds of grids by their central differences: CC_AXES an identity direction with every 1 / spacing
+// a float32 (1, 2, 0.5, 0.8 mm ...); CC_ROTATED another direction whose probes stay within one voxel
+// of theirs; CC_ANY any of these and the rest (0.9 mm, a rotated grid of very unequal spacings).
+enum CcMode { CC_ANY, CC_AXES, CC_ROTATED };
 
 struct CcArgs {
     DevGrid g;
     long long ps;       // plane stride of the derivative fields
     int zchunk;         // slices per CTA
     int identity_dir;   // direction is the identity: axis-aligned probes
-    double probe[3][3]; // index offset of +half a spacing along physical axis d: probe[d][r]
+    int stencil;        // rotated grid whose probes stay within one voxel: `probe` holds them
     double isp[3];      // 1 / spacing (the central difference's denominator)
+    float ispf[3];      // the same in float32
+    int mode;           // the kernel's MODE
+    // the probe at -half (p = 2d) and +half (2d + 1) a spacing along physical axis d, relative to
+    // its voxel: index offset of its lower corner (-1 or 0) and weights of the upper one
+    signed char base[6][3];
+    float weight[6][3];
 };
 
-// Shared-memory layout (dynamic): the z-window sums of every halo column, [5][HY*HX] double
-// (+ [HY*HX] int counts with a mask); y sums [5][HX][TY+1] double, column-major with an odd
-// column stride (+ [TY][HX] int counts); the raw voxels of the tile with a one-voxel halo for the
-// last D slices, [D][TY+2][TX+2] float2 (f, m), for the centre values and the central
-// differences; the x sums of the tile's voxels [5][TX][TY+1] double; block-reduction space.
-// The odd strides keep every pass free of bank conflicts: the y pass stores consecutive columns,
-// the x pass reads eight rows of two column groups per half-warp, and each voxel's thread reads
-// its own row of a column.
+// Shared-memory layout (dynamic): the z-window sums of every halo column, [5][HY][HX] double
+// (+ [HY][HX] int counts with a mask); y sums [5][HX][TY+1] double, column-major with an odd
+// column stride (+ [TY][HX] int counts); the x sums of the tile's voxels [5][TX][TY+1] double; the
+// raw voxels of the tile with a one-voxel halo for four slices, [4][TY+2][TX+2] float2 (f, m), for
+// the central differences; block-reduction space. The odd strides keep every pass free of bank
+// conflicts: the y pass stores consecutive columns, the x pass reads consecutive rows, and each
+// voxel's thread reads its own row of a column.
 template <int R, int TY, bool MK>
 struct Layout {
     static constexpr int HX = TX + 2 * R;
     static constexpr int HY = TY + 2 * R;
     static constexpr int HC = HX * HY;           // halo columns of the tile
-    static constexpr int NT = TX * TY;
+    static constexpr int NT = CC_NT;
     static constexpr int CPT = (HC + NT - 1) / NT;  // halo columns per thread
     static constexpr int NP = MK ? 4 : 3;  // block partials: cc, |dF|^2, |dM|^2 (+ valid voxels)
     static constexpr int RX = TX + 2, RY = TY + 2, RXY = RX * RY;
-    // raw slices kept: the output at step k reads slices k-R-1 .. k-R+1, and slice k is written
-    // before step k's first barrier, while slow threads may still read step k-1's outputs
-    static constexpr int D = R + 3;
+    static constexpr int RING = RXY - TX * TY;   // raw voxels around the tile, one a thread
+    static constexpr int D = 4;                  // raw slices: z - 1, z, z + 1 and the next one
+    static constexpr int YS = TY + 1;            // odd: TY is even
+    static constexpr int GX = 8;                 // outputs of an item of the x pass
+    static constexpr int YI = 5 * HX, XI = 5 * TY * (TX / GX);  // items of the y and x passes
+    static_assert(TX % GX == 0 && RING <= NT && YI <= NT && XI <= NT && TX * TY == NT,
+                  "one item a thread");
     static constexpr size_t zs1 = sizeof(double) * 5 * HC + (MK ? sizeof(int) * HC : 0);
-    static constexpr int YS = TY + 1;                                  // odd: TY is even
-    static constexpr int XG = 8;                                       // x outputs per item
-    static_assert(TX % XG == 0, "whole x groups");
     static constexpr size_t xs_bytes = sizeof(double) * 5 * HX * YS;  // y sums [5][HX][YS]
     static constexpr size_t xc_bytes = MK ? sizeof(int) * TY * HX : 0;
     static constexpr size_t raw_bytes = sizeof(float2) * D * RXY;
@@ -79,14 +101,9 @@ struct Layout {
 // shared memory, where the y pass reads them) one slice per step: the entering slice is added
 // and the leaving slice (read again, from L2) subtracted -- before the step's first barrier, which
 // the previous step's y pass has passed. Products of float32 voxels are exact in float64, so the
-// running sums carry no drift beyond float64 rounding. The y pass makes column sums of them four
-// output rows at a time, the x pass eight outputs of a row at a time, and each thread then reads
-// its own voxel's window sums. The kernel is bound by shared-memory bandwidth, which this order spends
-// least on: the shared-tap pairs sit in the pass over the wider (halo) extent, and both passes
-// read along consecutive banks.
-#ifndef FW_CC_MIN_BLOCKS
-#define FW_CC_MIN_BLOCKS 3
-#endif
+// running sums carry no drift beyond float64 rounding. The y and x passes make eight outputs an
+// item, and each thread then reads its own voxel's window sums.
+constexpr int CC_MIN_BLOCKS = 3;
 
 // The window sums' arithmetic. SumF64 (the default): float64, in which the products of float32
 // voxels are exact. SumC32: compensated float32, a (hi, lo) float pair per sum -- products split
@@ -136,9 +153,48 @@ struct SumC32 {
     __device__ static __forceinline__ double value(T a) { return (double)a.x + (double)a.y; }
 };
 
+// The G sums of 2R + 1 consecutive values out of G + 2R (load(t), t = 0 ..), store(j, sum of
+// load(j) .. load(j + 2R)), without a subtraction: the windows of GS neighbouring outputs all
+// contain the values GS-1 .. 2R, so each is a suffix sum that ends at 2R plus a prefix sum that
+// starts at 2R + 1 (van Herk's and Gil and Werman's running extremum, for sums): about 2.7 additions
+// an output at R = 4 in place of 8. A window of zeros sums to exactly zero.
+template <class Acc, int R, int G, class Load, class Store>
+__device__ __forceinline__ void window_sums(Load load, Store store) {
+    using T = typename Acc::T;
+    constexpr int GS = R == 1 ? 2 : (R <= 3 ? 4 : 8);  // GS <= 2R + 1
+    static_assert(G % GS == 0, "whole groups");
+#pragma unroll
+    for (int h = 0; h < G; h += GS) {
+        T s[GS];
+        T c = load(h + GS - 1);
+#pragma unroll
+        for (int t = GS; t <= 2 * R; ++t) c = Acc::add(c, load(h + t));
+        s[GS - 1] = c;
+#pragma unroll
+        for (int j = GS - 2; j >= 0; --j) s[j] = Acc::add(s[j + 1], load(h + j));
+        store(h, s[0]);
+        T p = load(h + 2 * R + 1);
+        store(h + 1, Acc::add(s[1], p));
+#pragma unroll
+        for (int j = 2; j < GS; ++j) {
+            p = Acc::add(p, load(h + 2 * R + j));
+            store(h + j, Acc::add(s[j], p));
+        }
+    }
+}
+
+// The exact probes of a rotated grid's faces, called rather than inlined: their float64 registers
+// would be spilled for in the tile's loop.
+__device__ __noinline__ void cc_exact_gradient(const float* __restrict__ img, const DevGrid& g,
+                                               int x, int y, int z, float out[3]) {
+    central_difference_exact(img, g, x, y, z, out);
+}
+
 // One tile (bx, by, bz) of the CC pair: writes the tile's derivative voxels and leaves the
-// thread's sums [cc, |dF|^2, |dM|^2, valid voxels] in acc_out.
-template <int R, int TY, bool MK, class Acc = SumF64>
+// thread's sums [cc, |dF|^2, |dM|^2, valid voxels] in acc_out. MODE: how the central differences
+// are formed, ANY grid's, or one of the two usual kinds alone (registers that the other kinds need
+// would be spilled for in the loop).
+template <int R, int TY, bool MK, int MODE, class Acc = SumF64>
 __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
                                         unsigned char* smem, const float* __restrict__ fimg,
                                         const float* __restrict__ mimg,
@@ -148,6 +204,8 @@ __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
     using L = Layout<R, TY, MK>;
     using T = typename Acc::T;
     static_assert(sizeof(T) == sizeof(double), "a window sum takes 8 bytes");
+    T* zs = reinterpret_cast<T*>(smem);
+    int* zc = reinterpret_cast<int*>(zs + 5 * L::HC);
     T* xs = reinterpret_cast<T*>(smem + L::zs1);
     int* xc = reinterpret_cast<int*>(smem + L::zs1 + L::xs_bytes);
     float2* raw = reinterpret_cast<float2*>(smem + L::zs1 + L::xs_bytes + L::xc_bytes);
@@ -164,184 +222,258 @@ __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
     const long long sxy = (long long)nx * ny;
 
     double acc_cc = 0.0, acc_nf = 0.0, acc_nm = 0.0, acc_nv = 0.0;
-    // analytic voxel counts of the clamped window along x and y
-    const int cxn = own ? (min(x + R, nx - 1) - max(x - R, 0) + 1) : 0;
-    const int cyn = own ? (min(y + R, ny - 1) - max(y - R, 0) + 1) : 0;
 
-    // the thread's halo columns: offset inside a slice, -1 outside the image (sums stay zero)
-    // and, for columns within one voxel of the tile, their slot in a raw slice (-1 otherwise)
-    int coff[L::CPT], ridx[L::CPT];
-    T* zs = reinterpret_cast<T*>(smem);
-    int* zc = reinterpret_cast<int*>(zs + 5 * L::HC);
+    // the thread's halo columns: offset inside a slice, OUT outside the image (sums stay zero)
+    constexpr unsigned int OUT = 0xffffffffu;
+    unsigned int coff[L::CPT];
 #pragma unroll
     for (int j = 0; j < L::CPT; ++j) {
         const int s = tid + j * L::NT;
-        coff[j] = -1;
-        ridx[j] = -1;
+        coff[j] = OUT;
         if (s < L::HC) {
             const int hy = s / L::HX, hx = s - hy * L::HX;
             const int gx = x0 - R + hx, gy = y0 - R + hy;
             if (gx >= 0 && gx < nx && gy >= 0 && gy < ny) coff[j] = gy * nx + gx;
-            const int rx = hx - (R - 1), ry = hy - (R - 1);
-            if (rx >= 0 && rx < L::RX && ry >= 0 && ry < L::RY) ridx[j] = ry * L::RX + rx;
-        }
-        if (s < L::HC) {
-#pragma unroll
-            for (int q = 0; q < 5; ++q) zs[q * L::HC + s] = Acc::zero();
-            if constexpr (MK) zc[s] = 0;
         }
     }
-    // Non-zero voxels of each halo column's z window, fixed in the low byte, moving in the next
-    // (exact integers, never negative). The reference forms every window sum directly from the
-    // window's voxels (metric/cc.rs:137-157), so a window where an image is zero sums to exactly
-    // zero and its CC takes the degenerate value; a running sum keeps a float64 rounding residue
-    // of what entered and left, so the sums of an image are reset to zero whenever its count is.
-    int nzc[L::CPT];
+    // The last slice where each halo column of an image was not zero. The reference forms every
+    // window sum directly from the window's voxels (metric/cc.rs:137-157), so a window where an
+    // image is zero sums to exactly zero and its CC takes the degenerate value; a running sum keeps
+    // a float64 rounding residue of what entered and left, so an image's sums are reset to zero
+    // whenever its last non-zero slice is out of the window.
+    int lastf[L::CPT], lastm[L::CPT];
+    const int kb = max(z0 - R, 0);
+    // the first window's slices but the last: additions only, their loads in flight together
+    {
+        T zsum[L::CPT][5];
+        int cnt[L::CPT];
 #pragma unroll
-    for (int j = 0; j < L::CPT; ++j) nzc[j] = 0;
+        for (int j = 0; j < L::CPT; ++j) {
+            lastf[j] = lastm[j] = kb - 2 * R - 2;
+            cnt[j] = 0;
+#pragma unroll
+            for (int q = 0; q < 5; ++q) zsum[j][q] = Acc::zero();
+        }
+        const int ke = min(z0 + R, nz);
+#pragma unroll 4
+        for (int k = kb; k < ke; ++k) {
+            const long long zi = (long long)k * sxy;
+#pragma unroll
+            for (int j = 0; j < L::CPT; ++j) {
+                float f = 0.0f, m = 0.0f;
+                if (coff[j] != OUT) {
+                    f = __ldg((fimg + zi) + coff[j]);
+                    m = __ldg((mimg + zi) + coff[j]);
+                    if constexpr (MK) {
+                        const bool v = __ldg((vimg + zi) + coff[j]) != 0.0f;
+                        if (!v) f = m = 0.0f;  // a masked-out voxel adds nothing
+                        cnt[j] += (int)v;
+                    }
+                }
+                if (f != 0.0f) lastf[j] = k;
+                if (m != 0.0f) lastm[j] = k;
+                zsum[j][0] = Acc::add(zsum[j][0], Acc::diff(f, 0.0f));
+                zsum[j][1] = Acc::add(zsum[j][1], Acc::diff(m, 0.0f));
+                zsum[j][2] = Acc::add(zsum[j][2], Acc::prod_diff(f, f, 0.0f, 0.0f));
+                zsum[j][3] = Acc::add(zsum[j][3], Acc::prod_diff(m, m, 0.0f, 0.0f));
+                zsum[j][4] = Acc::add(zsum[j][4], Acc::prod_diff(f, m, 0.0f, 0.0f));
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < L::CPT; ++j) {
+            const int s = tid + j * L::NT;
+            if (s < L::HC) {
+#pragma unroll
+                for (int q = 0; q < 5; ++q) zs[q * L::HC + s] = zsum[j][q];
+                if constexpr (MK) zc[s] = cnt[j];
+            }
+        }
+    }
     // entering slice k and leaving slice k - 2R - 1 of the next step, in flight during a step
     float2 pin[L::CPT], pout[L::CPT];
     bool vin[L::CPT], vout[L::CPT];
-    const int kb = max(z0 - R, 0);
     auto fetch = [&](int k) {
         const bool add = k < nz, sub = k - 2 * R - 1 >= kb;
         const long long zi = (long long)k * sxy, zo = (long long)(k - 2 * R - 1) * sxy;
+        const float *fi = fimg + zi, *mi = mimg + zi, *fo = fimg + zo, *mo = mimg + zo;
 #pragma unroll
         for (int j = 0; j < L::CPT; ++j) {
-            const bool c = coff[j] >= 0;
-            pin[j] = c && add ? make_float2(__ldg(fimg + zi + coff[j]), __ldg(mimg + zi + coff[j]))
+            const bool c = coff[j] != OUT;
+            pin[j] = c && add ? make_float2(__ldg(fi + coff[j]), __ldg(mi + coff[j]))
                               : make_float2(0.0f, 0.0f);
-            pout[j] = c && sub ? make_float2(__ldg(fimg + zo + coff[j]), __ldg(mimg + zo + coff[j]))
+            pout[j] = c && sub ? make_float2(__ldg(fo + coff[j]), __ldg(mo + coff[j]))
                                : make_float2(0.0f, 0.0f);
-            if constexpr (MK) {  // pin stays raw: the central differences read it
-                vin[j] = c && add && __ldg(vimg + zi + coff[j]) != 0.0f;
-                vout[j] = c && sub && __ldg(vimg + zo + coff[j]) != 0.0f;
+            if constexpr (MK) {
+                vin[j] = c && add && __ldg((vimg + zi) + coff[j]) != 0.0f;
+                vout[j] = c && sub && __ldg((vimg + zo) + coff[j]) != 0.0f;
+                if (!vin[j]) pin[j] = make_float2(0.0f, 0.0f);
                 if (!vout[j]) pout[j] = make_float2(0.0f, 0.0f);
             }
         }
     };
-    fetch(kb);
-    for (int k = kb; k < z1 + R; ++k) {
-        // z step: add slice k (if it exists), drop slice k - 2R - 1 (if it was added)
-        float2* rslot = raw + (k % L::D) * L::RXY;
+    // the raw voxels of the tile and its one-voxel ring, clamped at the image's faces: the thread's
+    // own voxel's column (also kept in registers) and, for the first RING threads, one of the ring
+    const unsigned int ocol = (unsigned int)(min(y, ny - 1) * nx + min(x, nx - 1));
+    unsigned int rcol = 0;
+    int rslot = 0;
+    if (tid < L::RING) {
+        int rx, ry;
+        if (tid < 2 * L::RX) {
+            ry = tid < L::RX ? 0 : L::RY - 1;
+            rx = tid < L::RX ? tid : tid - L::RX;
+        } else {
+            const int t = tid - 2 * L::RX;
+            ry = 1 + (t >> 1);
+            rx = (t & 1) ? L::RX - 1 : 0;
+        }
+        rslot = ry * L::RX + rx;
+        rcol = (unsigned int)(min(max(y0 - 1 + ry, 0), ny - 1) * nx + min(max(x0 - 1 + rx, 0), nx - 1));
+    }
+    const int oslot = (ty + 1) * L::RX + tx + 1;
+    auto voxel = [&](int z, unsigned int col) {
+        const long long o = (long long)min(max(z, 0), nz - 1) * sxy;
+        return make_float2(__ldg((fimg + o) + col), __ldg((mimg + o) + col));
+    };
+    float2 lo, cur = voxel(z0 - 1, ocol), hi = voxel(z0, ocol);  // shifted by the first step
+    float2 nown = voxel(z0 + 1, ocol), nring = make_float2(0.0f, 0.0f);
+    raw[((z0 - 1) & 3) * L::RXY + oslot] = cur;
+    raw[(z0 & 3) * L::RXY + oslot] = hi;
+    if (tid < L::RING) {
+        raw[((z0 - 1) & 3) * L::RXY + rslot] = voxel(z0 - 1, rcol);
+        raw[(z0 & 3) * L::RXY + rslot] = voxel(z0, rcol);
+        nring = voxel(z0 + 1, rcol);
+    }
+    const T* own_sums = sx + tx * L::YS + ty;
+    // identity grids: whether the probes of the faces are inside (a coordinate's probes do not
+    // depend on the others): bit 0 x, bits 1 and 2 the first and last slice, bit 3 y
+    unsigned int ok = ~0u;
+    if ((MODE == CC_AXES || (MODE == CC_ANY && a.identity_dir)) && own) {
+        auto inside = [&](int i, int j, int k, int d, int n) {
+            return axis_probe_inside(a.g, i, j, k, d, -1.0, n) && axis_probe_inside(a.g, i, j, k, d, +1.0, n);
+        };
+        if (!inside(x, y0, z0, 0, nx)) ok &= ~1u;
+        if (!inside(x, y0, 0, 2, nz)) ok &= ~2u;
+        if (!inside(x, y0, nz - 1, 2, nz)) ok &= ~4u;
+        if (!inside(x, y, z0, 1, ny)) ok &= ~8u;
+    }
+    // analytic voxel count of the clamped window along x and y
+    const int cxy = own ? (min(x + R, nx - 1) - max(x - R, 0) + 1) *
+                              (min(y + R, ny - 1) - max(y - R, 0) + 1) : 1;
+    int pcnt = 0;
+    double icnt = 0.0;
+    fetch(z0 + R);
+    for (int z = z0; z < z1; ++z) {
+        // the raw slice z + 1, then the z step: add slice k = z + R (if it exists), drop slice
+        // k - 2R - 1 (if it was added)
+        lo = cur;
+        cur = hi;
+        hi = nown;
+        {
+            float2* slot = raw + ((z + 1) & 3) * L::RXY;
+            slot[oslot] = nown;
+            if (tid < L::RING) slot[rslot] = nring;
+        }
 #pragma unroll
         for (int j = 0; j < L::CPT; ++j) {
-            if (ridx[j] >= 0 && k < nz) rslot[ridx[j]] = pin[j];
-            float2 a = pin[j];
-            if constexpr (MK)
-                if (!vin[j]) a = make_float2(0.0f, 0.0f);  // a masked-out voxel adds nothing
-            const float f = a.x, m = a.y, g = pout[j].x, n = pout[j].y;
+            const float f = pin[j].x, m = pin[j].y, g = pout[j].x, n = pout[j].y;
             const int s = tid + j * L::NT;
             if (s < L::HC) {
-                T* zq = zs + s;
-                nzc[j] += ((int)(f != 0.0f) - (int)(g != 0.0f)) +
-                          256 * ((int)(m != 0.0f) - (int)(n != 0.0f));
-                const bool fz = (nzc[j] & 255) == 0, mz = (nzc[j] >> 8) == 0;
-                zq[0] = fz ? Acc::zero() : Acc::add(zq[0], Acc::diff(f, g));
-                zq[L::HC] = mz ? Acc::zero() : Acc::add(zq[L::HC], Acc::diff(m, n));
-                zq[2 * L::HC] = fz ? Acc::zero() : Acc::add(zq[2 * L::HC], Acc::prod_diff(f, f, g, g));
-                zq[3 * L::HC] = mz ? Acc::zero() : Acc::add(zq[3 * L::HC], Acc::prod_diff(m, m, n, n));
-                zq[4 * L::HC] = (fz || mz) ? Acc::zero()
-                                           : Acc::add(zq[4 * L::HC], Acc::prod_diff(f, m, g, n));
+                // four zeros change nothing (the sums of a zero background are left alone)
+                if (((__float_as_uint(f) | __float_as_uint(m) | __float_as_uint(g) |
+                      __float_as_uint(n)) << 1) != 0u) {
+                    T* zq = zs + s;
+                    if (f != 0.0f) lastf[j] = z + R;
+                    if (m != 0.0f) lastm[j] = z + R;
+                    T v0 = Acc::add(zq[0], Acc::diff(f, g));
+                    T v1 = Acc::add(zq[L::HC], Acc::diff(m, n));
+                    T v2 = Acc::add(zq[2 * L::HC], Acc::prod_diff(f, f, g, g));
+                    T v3 = Acc::add(zq[3 * L::HC], Acc::prod_diff(m, m, n, n));
+                    T v4 = Acc::add(zq[4 * L::HC], Acc::prod_diff(f, m, g, n));
+                    if (min(lastf[j], lastm[j]) < z - R) {
+                        if (lastf[j] < z - R) v0 = v2 = Acc::zero();
+                        if (lastm[j] < z - R) v1 = v3 = Acc::zero();
+                        v4 = Acc::zero();
+                    }
+                    zq[0] = v0;
+                    zq[L::HC] = v1;
+                    zq[2 * L::HC] = v2;
+                    zq[3 * L::HC] = v3;
+                    zq[4 * L::HC] = v4;
+                }
                 if constexpr (MK) zc[s] += (int)vin[j] - (int)vout[j];
             }
         }
-        if (k + 1 < z1 + R) fetch(k + 1);
-        const int z = k - R;
-        if (z < z0) continue;  // the window is still filling (uniform across the CTA)
-
+        if (z + 1 < z1) {
+            fetch(z + 1 + R);
+            nown = voxel(z + 2, ocol);
+            if (tid < L::RING) nring = voxel(z + 2, rcol);
+        }
         __syncthreads();  // z sums visible; the previous x pass is done with the y sums
-        // y pass: each item makes four output rows of one halo column for one of the five window
-        // sums from one window of 2r + 4 rows, as two pairs of adjacent rows whose 2r middle rows are
-        // shared (each pair's sums in the same order as alone); a warp's items are consecutive
-        // columns, so its loads and stores fall on distinct banks
-        static_assert(TY % 4 == 0, "the y pass makes output rows in fours");
-        for (int s = tid; s < 5 * L::HX * (TY / 4); s += L::NT) {
-            const int q = s / (L::HX * (TY / 4)), rr = s - q * (L::HX * (TY / 4));
-            const int rq = rr / L::HX, hx = rr - rq * L::HX;
-            const T* col = zs + q * L::HC + 4 * rq * L::HX + hx;
-            T v[2 * R + 4];
+        // y pass: each item makes eight output rows of one halo column for one of the five window
+        // sums; a warp's items are consecutive columns, so its loads and stores fall on distinct
+        // banks
+        if (tid < L::YI) {
+            const int q = tid / L::HX, hx = tid - q * L::HX;
+            const T* col = zs + q * L::HC + hx;
+            T* o = xs + tid * L::YS;
+            window_sums<Acc, R, TY>([&](int t) { return col[t * L::HX]; },
+                                    [&](int j, T v) { o[j] = v; });
+        }
+        if constexpr (MK) {
+            for (int s = tid; s < L::HX * TY; s += L::NT) {
+                const int row = s / L::HX, hx = s - row * L::HX;
+                int cn = 0;
 #pragma unroll
-            for (int t = 0; t < 2 * R + 4; ++t) v[t] = col[t * L::HX];
-            T* o = xs + (q * L::HX + hx) * L::YS + 4 * rq;
-#pragma unroll
-            for (int p2 = 0; p2 < 4; p2 += 2) {
-                T c = Acc::zero(), e = Acc::zero();  // two partial sums: half-length add chains
-#pragma unroll
-                for (int t = 1; t <= 2 * R; t += 2) {
-                    c = Acc::add(c, v[p2 + t]);
-                    e = Acc::add(e, v[p2 + t + 1]);
-                }
-                c = Acc::add(c, e);
-                o[p2] = Acc::add(c, v[p2]);
-                o[p2 + 1] = Acc::add(c, v[p2 + 2 * R + 1]);
-            }
-            if constexpr (MK) {
-                if (q == 0) {
-                    const int* ccol = zc + 4 * rq * L::HX + hx;
-#pragma unroll
-                    for (int p2 = 0; p2 < 4; p2 += 2) {
-                        int cn = 0;
-#pragma unroll
-                        for (int t = 1; t <= 2 * R; ++t) cn += ccol[(p2 + t) * L::HX];
-                        xc[(4 * rq + p2) * L::HX + hx] = cn + ccol[p2 * L::HX];
-                        xc[(4 * rq + p2 + 1) * L::HX + hx] = cn + ccol[(p2 + 2 * R + 1) * L::HX];
-                    }
-                }
+                for (int t = 0; t <= 2 * R; ++t) cn += zc[(row + t) * L::HX + hx];
+                xc[s] = cn;
             }
         }
         __syncthreads();
-        // x pass: each item makes the sums of XG consecutive outputs of one row from one window
-        // of XG + 2r columns (each output's sum in the same order as alone: even taps, odd taps,
-        // the last); a half-warp's items are eight rows of two column groups
-        for (int s = tid; s < 5 * TY * (TX / L::XG); s += L::NT) {
-            const int q = s / (TY * (TX / L::XG)), rr = s - q * (TY * (TX / L::XG));
+        // x pass: each item makes eight consecutive outputs of one row; a warp's items are the
+        // rows of one column group, then of the next
+        if (tid < L::XI) {
+            const int q = tid / (TY * (TX / L::GX)), rr = tid - q * (TY * (TX / L::GX));
             const int row = rr % TY, g = rr / TY;
-            const T* in = xs + (q * L::HX + g * L::XG) * L::YS + row;
-            T v[L::XG + 2 * R];
-#pragma unroll
-            for (int t = 0; t < L::XG + 2 * R; ++t) v[t] = in[t * L::YS];
-            T* out = sx + (q * TX + g * L::XG) * L::YS + row;
-#pragma unroll
-            for (int j = 0; j < L::XG; ++j) {
-                T e = Acc::zero(), o = Acc::zero();
-#pragma unroll
-                for (int t = 0; t < 2 * R; t += 2) {
-                    e = Acc::add(e, v[j + t]);
-                    o = Acc::add(o, v[j + t + 1]);
-                }
-                out[j * L::YS] = Acc::add(Acc::add(e, o), v[j + 2 * R]);
-            }
+            const T* in = xs + (q * L::HX + g * L::GX) * L::YS + row;
+            T* out = sx + (q * TX + g * L::GX) * L::YS + row;
+            window_sums<Acc, R, L::GX>([&](int t) { return in[t * L::YS]; },
+                                       [&](int j, T v) { out[j * L::YS] = v; });
         }
         __syncthreads();
         if (!own) continue;
         double S[5];
 #pragma unroll
-        for (int q = 0; q < 5; ++q) S[q] = Acc::value(sx[(q * TX + tx) * L::YS + ty]);
+        for (int q = 0; q < 5; ++q) S[q] = Acc::value(own_sums[q * TX * L::YS]);
 
         // ---- output voxel (x, y, z) ----
-        const long long l = (long long)z * sxy + (long long)y * nx + x;
+        const long long slice = (long long)z * sxy;
+        float *pf = d_fixed + slice, *pm = d_moving + slice;
         double cnt;
         if constexpr (MK) {
-            if (__ldg(vimg + l) == 0.0f) {
-                d_fixed[l] = d_fixed[l + a.ps] = d_fixed[l + 2 * a.ps] = 0.0f;
-                d_moving[l] = d_moving[l + a.ps] = d_moving[l + 2 * a.ps] = 0.0f;
+            if (__ldg((vimg + slice) + ocol) == 0.0f) {
+                pf[ocol] = (pf + a.ps)[ocol] = (pf + 2 * a.ps)[ocol] = 0.0f;
+                pm[ocol] = (pm + a.ps)[ocol] = (pm + 2 * a.ps)[ocol] = 0.0f;
                 continue;
             }
             int Sc = 0;
 #pragma unroll
             for (int t = 0; t <= 2 * R; ++t) Sc += xc[ty * L::HX + tx + t];
             cnt = (double)Sc;  // >= 1: the centre is valid
+            icnt = 1.0 / cnt;
             acc_nv += 1.0;
         } else {
-            const int czn = min(z + R, nz - 1) - max(z - R, 0) + 1;
-            cnt = (double)(cxn * cyn * czn);
+            const int c = cxy * (min(z + R, nz - 1) - max(z - R, 0) + 1);
+            cnt = (double)c;
+            if (c != pcnt) {  // changes near the z faces only
+                icnt = 1.0 / cnt;
+                pcnt = c;
+            }
         }
-        const float2* cs = raw + (z % L::D) * L::RXY + (ty + 1) * L::RX + (tx + 1);
-        const float fv = cs[0].x, mv = cs[0].y;
+        const float2* cs = raw + (z & 3) * L::RXY + oslot;
+        const float2 centre = MODE == CC_ROTATED ? cs[0] : cur;
+        const float fv = centre.x, mv = centre.y;
         // metric/cc.rs:267-302 (same expression order)
         const double sum_f = S[0], sum_m = S[1], sum_f2 = S[2], sum_m2 = S[3], sum_fm = S[4];
-        const double icnt = 1.0 / cnt;
         const double fmean = sum_f * icnt, mmean = sum_m * icnt;
         const double s_ff = sum_f2 - fmean * sum_f - fmean * sum_f + cnt * fmean * fmean;
         const double s_mm = sum_m2 - mmean * sum_m - mmean * sum_m + cnt * mmean * mmean;
@@ -362,53 +494,69 @@ __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
         acc_cc += cc;
         // gradients of moving (for the first direction) and of fixed (for the second)
         float gm[3], gf[3];
-        if (a.identity_dir) {
+        if (MODE == CC_AXES || (MODE == CC_ANY && a.identity_dir)) {
             // interp.rs:96-120 on an identity-direction grid: the probes at +-half a spacing lerp
-            // halfway toward the neighbours along the axis, read from the raw slices
-            const int nn[3] = {nx, ny, nz};
-            const int pos[3] = {x, y, z};
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                gm[d] = 0.0f;
-                gf[d] = 0.0f;
-                if (!axis_probe_inside(a.g, x, y, z, d, -1.0, nn[d]) ||
-                    !axis_probe_inside(a.g, x, y, z, d, +1.0, nn[d]))
-                    continue;
-                const int p = pos[d];
-                float2 lo = cs[0], hi = cs[0];
-                if (d == 0) {
-                    if (p > 0) lo = cs[-1];
-                    if (p < nn[d] - 1) hi = cs[1];
-                } else if (d == 1) {
-                    if (p > 0) lo = cs[-L::RX];
-                    if (p < nn[d] - 1) hi = cs[L::RX];
+            // halfway toward the neighbours along the axis. Upper probe at p + 0.5: lerp to p + 1
+            // unless p is the last voxel; lower probe at p - 0.5: base p - 1 with weight 0.5, or
+            // the first voxel itself (a face's missing neighbour is the voxel itself here)
+            auto diff = [&](int d, bool in, float2 p, float2 q) {
+                const float m2 = fmaf(q.y - mv, 0.5f, mv), m1 = fmaf(mv - p.y, 0.5f, p.y);
+                const float f2 = fmaf(q.x - fv, 0.5f, fv), f1 = fmaf(fv - p.x, 0.5f, p.x);
+                if (MODE == CC_AXES) {  // the float64 product of two floats is exact: one rounding either way
+                    gm[d] = (m2 - m1) * a.ispf[d];
+                    gf[d] = (f2 - f1) * a.ispf[d];
                 } else {
-                    const int o = (ty + 1) * L::RX + (tx + 1);
-                    if (p > 0) lo = raw[((z - 1) % L::D) * L::RXY + o];
-                    if (p < nn[d] - 1) hi = raw[((z + 1) % L::D) * L::RXY + o];
+                    gm[d] = (float)((double)(m2 - m1) * a.isp[d]);
+                    gf[d] = (float)((double)(f2 - f1) * a.isp[d]);
                 }
-                // upper probe at p + 0.5: lerp to p + 1 unless p is the last voxel; lower probe
-                // at p - 0.5: base p - 1 with weight 0.5, or the first voxel itself
-                const float m2 = p < nn[d] - 1 ? fmaf(hi.y - mv, 0.5f, mv) : mv;
-                const float f2 = p < nn[d] - 1 ? fmaf(hi.x - fv, 0.5f, fv) : fv;
-                const float m1 = p > 0 ? fmaf(mv - lo.y, 0.5f, lo.y) : mv;
-                const float f1 = p > 0 ? fmaf(fv - lo.x, 0.5f, lo.x) : fv;
-                gm[d] = (float)((double)(m2 - m1) * a.isp[d]);
-                gf[d] = (float)((double)(f2 - f1) * a.isp[d]);
+                if (!in) gm[d] = gf[d] = 0.0f;
+            };
+            diff(0, ok & 1u, cs[-1], cs[1]);
+            diff(1, ok & 8u, cs[-L::RX], cs[L::RX]);
+            diff(2, (z > 0 || (ok & 2u)) && (z < nz - 1 || (ok & 4u)), lo, hi);
+        } else if ((MODE == CC_ROTATED || a.stencil) && x > 0 && x < nx - 1 && y > 0 && y < ny - 1 && z > 0 && z < nz - 1) {
+            // a rotated grid: off the faces every probe's corners and weights are the same
+            const float2* below = raw + ((z - 1) & 3) * L::RXY + oslot;
+            const float2* above = raw + ((z + 1) & 3) * L::RXY + oslot;
+            float2 v[2];
+#pragma unroll
+            for (int p = 0; p < 6; ++p) {
+                const float wx = a.weight[p][0], wy = a.weight[p][1], wz = a.weight[p][2];
+                const int at = a.base[p][0] + L::RX * a.base[p][1];
+                const int ox = wx > 0.0f ? 1 : 0, oy = wy > 0.0f ? L::RX : 0;
+                const bool low = a.base[p][2] < 0;
+                auto plane = [&](const float2* s) {
+                    const float2 v00 = s[at], v10 = s[at + ox], v01 = s[at + oy], v11 = s[at + oy + ox];
+                    const float fx0 = fmaf(v10.x - v00.x, wx, v00.x);
+                    const float fx1 = fmaf(v11.x - v01.x, wx, v01.x);
+                    const float mx0 = fmaf(v10.y - v00.y, wx, v00.y);
+                    const float mx1 = fmaf(v11.y - v01.y, wx, v01.y);
+                    return make_float2(fmaf(fx1 - fx0, wy, fx0), fmaf(mx1 - mx0, wy, mx0));
+                };
+                const float2 a0 = plane(low ? below : cs);
+                v[p & 1] = a0;
+                if (wz > 0.0f) {
+                    const float2 a1 = plane(low ? cs : above);
+                    v[p & 1] = make_float2(fmaf(a1.x - a0.x, wz, a0.x), fmaf(a1.y - a0.y, wz, a0.y));
+                }
+                if (p & 1) {
+                    gf[p >> 1] = (float)((double)(v[1].x - v[0].x) * a.isp[p >> 1]);
+                    gm[p >> 1] = (float)((double)(v[1].y - v[0].y) * a.isp[p >> 1]);
+                }
             }
         } else {
-            central_difference_exact(mimg, a.g, x, y, z, gm);
-            central_difference_exact(fimg, a.g, x, y, z, gf);
+            cc_exact_gradient(mimg, a.g, x, y, z, gm);
+            cc_exact_gradient(fimg, a.g, x, y, z, gf);
         }
         const float fcf = (float)cf, fcm = (float)cm;
         float dfx = fcf * gm[0], dfy = fcf * gm[1], dfz = fcf * gm[2];
         float dmx = fcm * gf[0], dmy = fcm * gf[1], dmz = fcm * gf[2];
-        d_fixed[l] = dfx;
-        d_fixed[l + a.ps] = dfy;
-        d_fixed[l + 2 * a.ps] = dfz;
-        d_moving[l] = dmx;
-        d_moving[l + a.ps] = dmy;
-        d_moving[l + 2 * a.ps] = dmz;
+        pf[ocol] = dfx;
+        (pf + a.ps)[ocol] = dfy;
+        (pf + 2 * a.ps)[ocol] = dfz;
+        pm[ocol] = dmx;
+        (pm + a.ps)[ocol] = dmy;
+        (pm + 2 * a.ps)[ocol] = dmz;
         if (want_norms) {
             acc_nf += (double)dfx * dfx + (double)dfy * dfy + (double)dfz * dfz;
             acc_nm += (double)dmx * dmx + (double)dmy * dmy + (double)dmz * dmz;
@@ -470,8 +618,8 @@ __device__ __forceinline__ void cc_finish(const double* partials, unsigned int n
     }
 }
 
-template <int R, int TY, bool MK, class Acc = SumF64>
-__global__ void __launch_bounds__(TX * TY, FW_CC_MIN_BLOCKS) k_cc_pair(CcArgs a, const float* __restrict__ fimg,
+template <int R, int TY, bool MK, int MODE, class Acc = SumF64>
+__global__ void __launch_bounds__(CC_NT, CC_MIN_BLOCKS) k_cc_pair(const __grid_constant__ CcArgs a, const float* __restrict__ fimg,
                                                      const float* __restrict__ mimg,
                                                      const float* __restrict__ vimg,
                                                      float* __restrict__ d_fixed,
@@ -484,7 +632,7 @@ __global__ void __launch_bounds__(TX * TY, FW_CC_MIN_BLOCKS) k_cc_pair(CcArgs a,
     extern __shared__ __align__(16) unsigned char smem[];
     double* red = reinterpret_cast<double*>(smem + L::red_off);
     double acc[4];
-    cc_tile<R, TY, MK, Acc>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem, fimg, mimg, vimg,
+    cc_tile<R, TY, MK, MODE, Acc>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem, fimg, mimg, vimg,
                             d_fixed, d_moving, want_norms, acc);
     // block partials, then the fixed-order last-block reduction
     const unsigned int nblocks = gridDim.x * gridDim.y * gridDim.z;
@@ -499,9 +647,9 @@ __global__ void __launch_bounds__(TX * TY, FW_CC_MIN_BLOCKS) k_cc_pair(CcArgs a,
 // its tile partials at partials + b * part_stride, its last-tile counter at counter[b] and its
 // [value, |dF|^2, |dM|^2] at result + b * result_stride. Tiles are summed in the single
 // kernel's block order, so a subject's value does not depend on the batch.
-template <int R, int TY>
-__global__ void __launch_bounds__(TX * TY, FW_CC_MIN_BLOCKS) k_cc_pair_batch(
-    CcArgs a, BatchList Lb, const float* __restrict__ fimg, const float* __restrict__ mimg,
+template <int R, int TY, int MODE>
+__global__ void __launch_bounds__(CC_NT, CC_MIN_BLOCKS) k_cc_pair_batch(
+    const __grid_constant__ CcArgs a, BatchList Lb, const float* __restrict__ fimg, const float* __restrict__ mimg,
     long long img_stride, float* __restrict__ d_fixed, float* __restrict__ d_moving,
     long long field_stride, double* __restrict__ partials, long long part_stride,
     unsigned int* __restrict__ counter, double* __restrict__ result, int result_stride,
@@ -516,7 +664,7 @@ __global__ void __launch_bounds__(TX * TY, FW_CC_MIN_BLOCKS) k_cc_pair_batch(
         int bx, by, bz;
         tile_coords(t, gx, gy, bx, by, bz);
         double acc[4];
-        cc_tile<R, TY, false>(a, bx, by, bz, smem, fimg + b * img_stride, mimg + b * img_stride,
+        cc_tile<R, TY, false, MODE>(a, bx, by, bz, smem, fimg + b * img_stride, mimg + b * img_stride,
                               nullptr, d_fixed + b * field_stride, d_moving + b * field_stride,
                               want_norms, acc);
         double* pb = partials + b * part_stride;
@@ -532,14 +680,14 @@ __global__ void __launch_bounds__(TX * TY, FW_CC_MIN_BLOCKS) k_cc_pair_batch(
 // CTAs (measured at the 193 x 229 x 193 finest level, r = 4: 8 chunks 0.398 ms, 5 chunks 0.401 ms,
 // 2 chunks -- less than one wave -- 0.426 ms), with chunks no thinner than 2R slices, the filling
 // steps every chunk pays before its first output.
-template <int R, int TY, bool MK, class Acc = SumF64>
+template <int R, int TY, bool MK, int MODE, class Acc = SumF64>
 int plan_launch(CcArgs& a, int num_sms, dim3* grid) {
     using L = Layout<R, TY, MK>;
-    FW_CUDA(cudaFuncSetAttribute(k_cc_pair<R, TY, MK, Acc>,
+    FW_CUDA(cudaFuncSetAttribute(k_cc_pair<R, TY, MK, MODE, Acc>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::bytes));
     static const int occ = [] {
         int o = 1;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_cc_pair<R, TY, MK, Acc>, L::NT,
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_cc_pair<R, TY, MK, MODE, Acc>, L::NT,
                                                           L::bytes) != cudaSuccess || o < 1)
             o = 1;
         return o;
@@ -556,16 +704,16 @@ int plan_launch(CcArgs& a, int num_sms, dim3* grid) {
     return 0;
 }
 
-template <int R, int TY, bool MK, class Acc = SumF64>
+template <int R, int TY, bool MK, int MODE, class Acc = SumF64>
 int launch_r(fw_ctx* ctx, const CcArgs& a0, const float* f, const float* m, const float* v,
              float* df, float* dm, double* d_result, int want_norms) {
     using L = Layout<R, TY, MK>;
     CcArgs a = a0;
     dim3 grid;
-    FW_TRY((plan_launch<R, TY, MK, Acc>(a, ctx->num_sms, &grid)));
+    FW_TRY((plan_launch<R, TY, MK, MODE, Acc>(a, ctx->num_sms, &grid)));
     unsigned int nblocks = grid.x * grid.y * grid.z;
     FW_TRY(ensure_scratch(ctx, SLOT_PARTIALS + (size_t)L::NP * nblocks + 16));
-    return launch_pdl(ctx, "k_cc_pair", k_cc_pair<R, TY, MK, Acc>, grid, dim3(L::NT), L::bytes,
+    return launch_pdl(ctx, "k_cc_pair", k_cc_pair<R, TY, MK, MODE, Acc>, grid, dim3(L::NT), L::bytes,
                       a, f, m, v, df, dm, ctx->d_scratch + SLOT_PARTIALS, ctx->d_counter + 1,
                       d_result, want_norms);
 }
@@ -580,9 +728,15 @@ int launch_radius(fw_ctx* ctx, const CcArgs& a, int radius, const float* f, cons
 #define FW_CC_RADIUS(RR)                                                                         \
     case RR:                                                                                    \
         if constexpr (!MK)                                                                      \
-            if (c32) return launch_r<RR, 8, false, SumC32>(ctx, a, f, m, v, df, dm, d_result,   \
-                                                          want_norms);                          \
-        return launch_r<RR, 8, MK>(ctx, a, f, m, v, df, dm, d_result, want_norms);
+            if (c32) return launch_r<RR, CC_TY, false, CC_ANY, SumC32>(ctx, a, f, m, v, df, dm,  \
+                                                                     d_result, want_norms);     \
+        if (a.mode == CC_AXES)                                                                  \
+            return launch_r<RR, CC_TY, MK, CC_AXES>(ctx, a, f, m, v, df, dm, d_result,          \
+                                                    want_norms);                                \
+        if (a.mode == CC_ROTATED)                                                               \
+            return launch_r<RR, CC_TY, MK, CC_ROTATED>(ctx, a, f, m, v, df, dm, d_result,       \
+                                                       want_norms);                             \
+        return launch_r<RR, CC_TY, MK, CC_ANY>(ctx, a, f, m, v, df, dm, d_result, want_norms);
     switch (radius) {
         FW_CC_RADIUS(1)
         FW_CC_RADIUS(2)
@@ -598,15 +752,15 @@ int launch_radius(fw_ctx* ctx, const CcArgs& a, int radius, const float* f, cons
 #undef FW_CC_RADIUS
 }
 
-template <int R>
+template <int R, int MODE>
 int launch_cc_batch_r(fw_ctx* ctx, const CcArgs& a, const BatchList& L, int blocks,
                       const float* f, const float* m, long long img_stride, float* df, float* dm,
                       long long field_stride, double* partials, long long part_stride,
                       unsigned int* counter, double* result, int result_stride, int want_norms) {
-    using Lay = Layout<R, 8, false>;
-    FW_CUDA(cudaFuncSetAttribute(k_cc_pair_batch<R, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)Lay::bytes));
-    k_cc_pair_batch<R, 8><<<blocks, Lay::NT, Lay::bytes, ctx->stream>>>(
+    using Lay = Layout<R, CC_TY, false>;
+    FW_CUDA(cudaFuncSetAttribute(k_cc_pair_batch<R, CC_TY, MODE>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes));
+    k_cc_pair_batch<R, CC_TY, MODE><<<blocks, Lay::NT, Lay::bytes, ctx->stream>>>(
         a, L, f, m, img_stride, df, dm, field_stride, partials, part_stride, counter, result,
         result_stride, want_norms);
     return check_launch(ctx, "k_cc_pair_batch");
@@ -614,11 +768,12 @@ int launch_cc_batch_r(fw_ctx* ctx, const CcArgs& a, const BatchList& L, int bloc
 
 template <int R>
 int cc_batch_occupancy() {
-    using Lay = Layout<R, 8, false>;
-    cudaFuncSetAttribute(k_cc_pair_batch<R, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)Lay::bytes);
+    using Lay = Layout<R, CC_TY, false>;
     int o = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_cc_pair_batch<R, 8>, Lay::NT,
+    if (cudaFuncSetAttribute(k_cc_pair_batch<R, CC_TY, CC_AXES>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)Lay::bytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_cc_pair_batch<R, CC_TY, CC_AXES>, Lay::NT,
                                                       Lay::bytes) != cudaSuccess || o < 1) {
         cudaGetLastError();
         o = 1;
@@ -631,18 +786,43 @@ CcArgs cc_args(const HostGrid& g, long long ps) {
     std::memset(&a, 0, sizeof(a));
     a.g = dev_grid(g);
     a.ps = ps;
-    for (int d = 0; d < 3; ++d) a.isp[d] = 1.0 / g.sp[d];
+    for (int d = 0; d < 3; ++d) {
+        a.isp[d] = 1.0 / g.sp[d];
+        a.ispf[d] = (float)a.isp[d];
+    }
     a.identity_dir = 1;
     for (int r = 0; r < 3; ++r)
         for (int c = 0; c < 3; ++c)
             if (g.dir[r * 3 + c] != (r == c ? 1.0 : 0.0)) a.identity_dir = 0;
+    const bool exact = (double)a.ispf[0] == a.isp[0] && (double)a.ispf[1] == a.isp[1] &&
+                       (double)a.ispf[2] == a.isp[2];
+    a.stencil = !a.identity_dir;
+    for (int p = 0; p < 6; ++p)
+        for (int r = 0; r < 3; ++r) {
+            // index offset along axis r of the probe along physical axis p / 2
+            const double h = (p & 1 ? 0.5 : -0.5) * g.sp[p / 2] * g.inv[r * 3 + p / 2];
+            double base = std::floor(h), w = h - base;
+            // within rounding of a voxel: that voxel (a probe's own rounding is this large)
+            if (w > 1.0 - 1e-12) {
+                base += 1.0;
+                w = 0.0;
+            } else if (w < 1e-12) {
+                w = 0.0;
+            }
+            if (!(base >= -1.0 && base + (w > 0.0 ? 1.0 : 0.0) <= 1.0)) a.stencil = 0;
+            else {
+                a.base[p][r] = (signed char)base;
+                a.weight[p][r] = (float)w;
+            }
+        }
+    a.mode = a.identity_dir ? (exact ? CC_AXES : CC_ANY) : (a.stencil ? CC_ROTATED : CC_ANY);
     return a;
 }
 
 }  // namespace
 
 int cc_batch_tiles(const HostGrid& g, int zchunk) {
-    const long long gx = (g.n[0] + TX - 1) / TX, gy = (g.n[1] + 7) / 8;
+    const long long gx = (g.n[0] + TX - 1) / TX, gy = (g.n[1] + CC_TY - 1) / CC_TY;
     const long long gz = (g.n[2] + zchunk - 1) / zchunk;
     return (int)(gx * gy * gz);
 }
@@ -671,9 +851,15 @@ int launch_cc_pair_batch(fw_ctx* ctx, const HostGrid& g, long long ps, int radiu
     a.zchunk = zchunk;
 #define FW_CC_BATCH(RR)                                                                          \
     case RR:                                                                                    \
-        return launch_cc_batch_r<RR>(ctx, a, L, blocks, fimg, mimg, img_stride, d_fixed,         \
-                                     d_moving, field_stride, partials, part_stride, counter,     \
-                                     result, result_stride, want_norms);
+        return a.mode == CC_AXES                                                                \
+                   ? launch_cc_batch_r<RR, CC_AXES>(ctx, a, L, blocks, fimg, mimg, img_stride,  \
+                                                    d_fixed, d_moving, field_stride, partials,  \
+                                                    part_stride, counter, result,               \
+                                                    result_stride, want_norms)                  \
+                   : launch_cc_batch_r<RR, CC_ANY>(ctx, a, L, blocks, fimg, mimg, img_stride,   \
+                                                   d_fixed, d_moving, field_stride, partials,   \
+                                                   part_stride, counter, result, result_stride, \
+                                                   want_norms);
     switch (radius) {
         FW_CC_BATCH(1)
         FW_CC_BATCH(2)
@@ -841,13 +1027,13 @@ int noalloc_scratch(int device, NoAllocScratch** out) {
     return 0;
 }
 
-template <int R, int TY>
+template <int R, int TY, int MODE>
 int noalloc_launch(const CcArgs& a0, int num_sms, const float* f, const float* m, float* df,
                    float* dm, double* result, NoAllocScratch* s, cudaStream_t stream) {
     using L = Layout<R, TY, false>;
     CcArgs a = a0;
     dim3 grid;
-    FW_TRY((plan_launch<R, TY, false>(a, num_sms, &grid)));
+    FW_TRY((plan_launch<R, TY, false, MODE>(a, num_sms, &grid)));
     long long nblocks = (long long)grid.x * grid.y * grid.z;
     if (nblocks > FW_NOALLOC_MAX_BLOCKS)
         return fail(FW_ERR_INVALID,
@@ -856,7 +1042,7 @@ int noalloc_launch(const CcArgs& a0, int num_sms, const float* f, const float* m
                         " the static scratch holds (use fw_cc_value_derivative_pair)");
     // the last-block counter must start at zero whatever the previous call left
     FW_CUDA(cudaMemsetAsync(s->counter, 0, sizeof(unsigned int), stream));
-    k_cc_pair<R, TY, false><<<grid, L::NT, L::bytes, stream>>>(a, f, m, nullptr, df, dm,
+    k_cc_pair<R, TY, false, MODE><<<grid, L::NT, L::bytes, stream>>>(a, f, m, nullptr, df, dm,
                                                                 s->partials, s->counter, result, 1);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "k_cc_pair (no alloc)");
@@ -881,26 +1067,26 @@ extern "C" int fw_cc_value_derivative_pair_noalloc(const fw_grid* grid, const fl
     FW_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device));
     NoAllocScratch* s = nullptr;
     FW_TRY(noalloc_scratch(device, &s));
-    CcArgs a;
-    std::memset(&a, 0, sizeof(a));
-    a.g = dev_grid(g);
-    a.ps = plane_stride;
-    for (int d = 0; d < 3; ++d) a.isp[d] = 1.0 / g.sp[d];
-    a.identity_dir = 1;
-    for (int r = 0; r < 3; ++r)
-        for (int c = 0; c < 3; ++c)
-            if (g.dir[r * 3 + c] != (r == c ? 1.0 : 0.0)) a.identity_dir = 0;
+    const CcArgs a = cc_args(g, plane_stride);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+#define FW_CC_NOALLOC(RR)                                                                        \
+    case RR:                                                                                    \
+        return a.mode == CC_AXES                                                                \
+                   ? noalloc_launch<RR, CC_TY, CC_AXES>(a, num_sms, fixed, moving, d_fixed,     \
+                                                        d_moving, result, s, st)                \
+                   : noalloc_launch<RR, CC_TY, CC_ANY>(a, num_sms, fixed, moving, d_fixed,      \
+                                                       d_moving, result, s, st);
     switch (radius) {
-        case 1: return noalloc_launch<1, 8>(a, num_sms, fixed, moving, d_fixed, d_moving, result, s, st);
-        case 2: return noalloc_launch<2, 8>(a, num_sms, fixed, moving, d_fixed, d_moving, result, s, st);
-        case 3: return noalloc_launch<3, 8>(a, num_sms, fixed, moving, d_fixed, d_moving, result, s, st);
-        case 4: return noalloc_launch<4, 8>(a, num_sms, fixed, moving, d_fixed, d_moving, result, s, st);
-        case 5: return noalloc_launch<5, 8>(a, num_sms, fixed, moving, d_fixed, d_moving, result, s, st);
-        case 6: return noalloc_launch<6, 8>(a, num_sms, fixed, moving, d_fixed, d_moving, result, s, st);
-        case 7: return noalloc_launch<7, 8>(a, num_sms, fixed, moving, d_fixed, d_moving, result, s, st);
-        case 8: return noalloc_launch<8, 8>(a, num_sms, fixed, moving, d_fixed, d_moving, result, s, st);
+        FW_CC_NOALLOC(1)
+        FW_CC_NOALLOC(2)
+        FW_CC_NOALLOC(3)
+        FW_CC_NOALLOC(4)
+        FW_CC_NOALLOC(5)
+        FW_CC_NOALLOC(6)
+        FW_CC_NOALLOC(7)
+        FW_CC_NOALLOC(8)
         default:
             return fail(FW_ERR_INVALID, "cc metric: radius must be in 1..=8 (BOX_RADIUS_MAX)");
     }
+#undef FW_CC_NOALLOC
 }

@@ -184,6 +184,32 @@ def test_cc_every_radius_path_matches(backend, radius):
     assert worst(backend.download_field(d2), e2) <= 1e-4 * np.abs(e2).max()
 
 
+@pytest.mark.parametrize("radius", [2, 3, 4, 7])
+@pytest.mark.parametrize("spacing,oblique", [((0.9, 0.9, 0.9), False), ((0.8, 2.0, 0.5), False),
+                                             ((1.1, 1.1, 1.1), True), ((0.5, 3.0, 0.7), True)])
+def test_cc_every_kind_of_grid_matches(backend, spacing, oblique, radius):
+    """The kernel's kinds of central differences: axis-aligned with a float32 1 / spacing and
+    without, rotated with probes within a voxel and beyond. Tiles of 32 x 8 with remainders on every
+    axis, a zero background and a masked pair."""
+    case = dict(CASES["awkward_oblique"], size=(67, 21, 27), spacing=spacing, radius=radius,
+                direction=CASES["awkward_oblique"]["direction"] if oblique else np.eye(3))
+    og, g = grid_of(case), fgrid(case)
+    fimg, mimg = image(case), image(case, seed_offset=3)
+    fimg[:, :, :20] = 0.0
+    mimg[:9] = 0.0
+    fi = backend.upload_image(g, fimg.astype(np.float32))
+    mi = backend.upload_image(g, mimg.astype(np.float32))
+    valid = ball_mask(case)
+    vi = backend.upload_image(g, valid.astype(np.float32))
+    for got, want in ((backend.cc_value_derivative_pair(fi, mi, radius),
+                       O.cc_pair(og, fimg, mimg, radius)),
+                      (backend.cc_value_derivative_pair_masked(fi, mi, vi, radius),
+                       O.cc_pair(og, fimg, mimg, radius, valid=valid))):
+        for (v, d), (w, e) in zip(got, want):
+            assert rel(v, w) <= 1e-5
+            assert worst(backend.download_field(d), e) <= 1e-4 * np.abs(e).max()
+
+
 def ball_mask(case):
     """metric/cc.rs:465-473's mask shape on the case grid: out of a ball, the first x plane and a
     corner strip; the inside value is 3 (any non-zero value counts)."""
