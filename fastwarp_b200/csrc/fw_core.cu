@@ -431,6 +431,27 @@ __global__ void __launch_bounds__(256) k_warp_t(WarpArgs a, int zchunk,
     warp_column(a, x, y, z0, z1, u, src, out);
 }
 
+// Two such warps onto one grid in one launch (the SyN iteration's fixed and moving sides): the
+// first gx x blocks are side 0's. Twice the blocks of one warp fill the SMs of the coarse levels
+// and leave one tail in place of two.
+struct WarpPair {
+    WarpArgs a[2];
+    const float* u[2];
+    const float* src[2];
+    float* out[2];
+};
+__global__ void __launch_bounds__(256) k_warp_pair(const __grid_constant__ WarpPair p, int zchunk,
+                                                   int gx) {
+    pdl_wait();
+    const int side = (int)blockIdx.x >= gx ? 1 : 0;
+    int x, y, z0, z1;
+    if (!column_of_tile(p.a[0].g.nx, p.a[0].g.ny, p.a[0].g.nz, zchunk, (int)blockIdx.x - side * gx,
+                        blockIdx.y, blockIdx.z, x, y, z0, z1))
+        return;
+    if (side == 0) warp_column(p.a[0], x, y, z0, z1, p.u[0], p.src[0], p.out[0]);
+    else warp_column(p.a[1], x, y, z0, z1, p.u[1], p.src[1], p.out[1]);
+}
+
 // The same warp for every active subject of a batch: subject b gathers from srcs[b] through
 // args[b] (per_subject) or from srcs[0] through args[0] (the shared template), with its field at
 // u + b * u_stride and its output at out + b * out_stride.
@@ -511,6 +532,27 @@ __global__ void __launch_bounds__(256) k_compose(FieldArgs a, int zchunk,
     int i, j, z0, z1;
     if (!column_of(a.g.nx, a.g.ny, a.g.nz, zchunk, i, j, z0, z1)) return;
     compose_column(a, i, j, z0, z1, u, w, out, max_bits, step);
+}
+
+// In place for both sides of a SyN iteration in one launch: field[s] composed with the update
+// u[s], scaled by step / its max at max_bits[s]; the first gx x blocks are side 0's.
+struct ComposePair {
+    FieldArgs a;
+    const float* u[2];
+    float* field[2];
+};
+__global__ void __launch_bounds__(256) k_compose_pair(const __grid_constant__ ComposePair p,
+                                                      int zchunk, int gx,
+                                                      const unsigned int* __restrict__ max_bits,
+                                                      double step) {
+    pdl_wait();
+    const int side = (int)blockIdx.x >= gx ? 1 : 0;
+    int i, j, z0, z1;
+    if (!column_of_tile(p.a.g.nx, p.a.g.ny, p.a.g.nz, zchunk, (int)blockIdx.x - side * gx, blockIdx.y,
+                        blockIdx.z, i, j, z0, z1))
+        return;
+    float* f = p.field[side];
+    compose_column(p.a, i, j, z0, z1, p.u[side], f, f, max_bits + side, step);
 }
 
 // In place for every active subject of a batch: field + b * stride composed with the update
@@ -761,6 +803,38 @@ int launch_compose(fw_ctx* ctx, const fw_field* disp, const fw_field* warping, f
     return launch_pdl(ctx, "k_compose", k_compose, grid, dim3(256), 0, a, zchunk,
                       (const float*)disp->d, (const float*)warping->d, out->d, d_scale_max_bits,
                       step);
+}
+
+int launch_warp_pair(fw_ctx* ctx, const fw_image* const src[2], const fw_field* const field[2],
+                     const fw_affine* const affine[2], float* const out[2]) {
+    WarpPair p;
+    for (int s = 0; s < 2; ++s) {
+        plain_warp_args(src[s]->grid, field[s]->grid, field[s]->ps, affine[s], p.a[s]);
+        p.u[s] = field[s]->d;
+        p.src[s] = src[s]->d;
+        p.out[s] = out[s];
+    }
+    int zchunk = 1;
+    dim3 grid = column_grid(p.a[0].g.nx, p.a[0].g.ny, p.a[0].g.nz, ctx->num_sms, &zchunk);
+    const int gx = (int)grid.x;
+    grid.x *= 2;
+    return launch_pdl(ctx, "k_warp_pair", k_warp_pair, grid, dim3(256), 0, p, zchunk, gx);
+}
+
+int launch_compose_pair(fw_ctx* ctx, const fw_field* const update[2], fw_field* const field[2],
+                        const unsigned int* d_max_bits, double step) {
+    ComposePair p;
+    p.a = FieldArgs{dev_grid(field[0]->grid), field[0]->ps};
+    for (int s = 0; s < 2; ++s) {
+        p.u[s] = update[s]->d;
+        p.field[s] = field[s]->d;
+    }
+    int zchunk = 1;
+    dim3 grid = column_grid(p.a.g.nx, p.a.g.ny, p.a.g.nz, ctx->num_sms, &zchunk);
+    const int gx = (int)grid.x;
+    grid.x *= 2;
+    return launch_pdl(ctx, "k_compose_pair", k_compose_pair, grid, dim3(256), 0, p, zchunk, gx,
+                      d_max_bits, step);
 }
 
 __global__ void k_image_product(const float* __restrict__ a, const float* __restrict__ b,

@@ -527,7 +527,7 @@ struct InvState {
     unsigned int lb;      // float bits: a lower bound on the running body's max error
     unsigned int ndefer;  // tiles whose update the running body left to the fix kernel
     float eps, limit;     // the last body's step and clamp (eps * max error)
-    int pad;
+    int run;              // whether the body in progress runs (the pair's bound kernel notes it)
 };
 
 // The inversion loop (fw_invert.cu). `res` (a field on the inverse's grid) keeps the residual
@@ -537,21 +537,28 @@ int enqueue_inversion_prefix(fw_ctx* ctx, const fw_field* field, fw_field* inver
                              cudaGraphConditionalHandle handle, int use_handle);
 int enqueue_inversion_body(fw_ctx* ctx, const fw_field* field, fw_field* inverse, fw_field* res,
                            InvState* st, cudaGraphConditionalHandle handle, int use_handle);
-// Graph mode: scratch for an inversion's bodies without the init kernel, and the inits of up to
-// kMaxInitHandles inversions (their states and WHILE conditions) in one kernel that also clears
-// zero[0..nzero).
-constexpr int kMaxInitHandles = 4;
+// One body of the same inversion of both sides of a SyN iteration in one launch of each kernel:
+// inverse[s] against field[s] with the state st[2 s]; a side whose loop has ended does nothing. With
+// use_handle the condition is set to whether either side runs another body.
+int enqueue_inversion_pair_body(fw_ctx* ctx, const fw_field* const field[2],
+                                fw_field* const inverse[2], fw_field* const res[2], InvState* st,
+                                cudaGraphConditionalHandle handle, int use_handle);
+int enqueue_inversion_pair_init(fw_ctx* ctx, const fw_invert_params& prm, InvState* st);
+// Graph mode: scratch for an inversion's bodies without the init kernel, and the inits of an
+// iteration's inversions (their states and up to kMaxInitHandles WHILE conditions) in one kernel that
+// also clears zero[0..nzero).
+constexpr int kMaxInitHandles = 2;
 int inversion_scratch(fw_ctx* ctx, const fw_field* field);
 int enqueue_inversion_inits(fw_ctx* ctx, InvState* st, int count, const fw_invert_params& prm,
-                            const cudaGraphConditionalHandle* handles, unsigned int* zero,
-                            int nzero);
+                            const cudaGraphConditionalHandle* handles, int nhandles,
+                            unsigned int* zero, int nzero);
 // One kernel of a body (0 bound, 1 step, 2 fix), for kernel timing.
 int enqueue_inversion_kernel(fw_ctx* ctx, const fw_field* field, fw_field* inverse, fw_field* res,
                              InvState* st, int which);
 long long inv_step_tiles(const HostGrid& g);
 // Warp parts of the step's tiles on grid g (the capacity of a deferred list).
 long long inv_step_parts(const HostGrid& g);
-// Scratch doubles an inversion on grid g needs (block partials and the deferred-tile list).
+// Scratch doubles two inversions on grid g need (each its block partials and deferred-tile list).
 size_t inv_scratch_doubles(const HostGrid& g);
 long long inv_bound_voxels(const HostGrid& g);
 // Adds a WHILE node on `handle` at the capture position of stream `s`; `body` receives the graph
@@ -744,6 +751,15 @@ int launch_image_product(fw_ctx* ctx, const fw_image* a, const fw_image* b, fw_i
 // out = warping + step/max * disp(x + warping) (step 1 without max bits).
 int launch_compose(fw_ctx* ctx, const fw_field* disp, const fw_field* warping, fw_field* out,
                    const unsigned int* d_scale_max_bits, double step);
+// The two sides of a SyN iteration in one launch each (fields of one grid and plane stride): the
+// plain warps; the smoothing of f[s] through tmp[s] with its max |u/sp| in d_max_bits[s] (the result
+// replaces f[s], or lies in tmp[s] when *in_tmp); the composition in place.
+int launch_warp_pair(fw_ctx* ctx, const fw_image* const src[2], const fw_field* const field[2],
+                     const fw_affine* const affine[2], float* const out[2]);
+int launch_smooth_pair(fw_ctx* ctx, fw_field* const f[2], fw_field* const tmp[2], double variance,
+                       unsigned int* d_max_bits, bool* in_tmp);
+int launch_compose_pair(fw_ctx* ctx, const fw_field* const update[2], fw_field* const field[2],
+                        const unsigned int* d_max_bits, double step);
 int launch_scale_by_max(fw_ctx* ctx, fw_field* f, const unsigned int* d_max_bits, double step);
 int invert_field(fw_ctx* ctx, const fw_field* field, fw_field* inverse,
                  const fw_invert_params& prm, fw_invert_stats* stats);

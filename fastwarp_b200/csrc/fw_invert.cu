@@ -166,6 +166,7 @@ __device__ __forceinline__ void init_state(InvState* __restrict__ st, const fw_i
     st->ndefer = 0u;
     st->eps = 0.0f;
     st->limit = 0.0f;
+    st->run = 0;
 }
 
 __global__ void k_inv_init(InvState* __restrict__ st, fw_invert_params prm,
@@ -174,20 +175,19 @@ __global__ void k_inv_init(InvState* __restrict__ st, fw_invert_params prm,
     if (use_handle) cudaGraphSetConditional(handle, st->go ? 1u : 0u);
 }
 
-// Several inversions' settings in one launch: states st[0..count) and the conditions of their
-// WHILE nodes; it also clears zero[0..nzero) (the SyN level graph begins every iteration with it:
-// its four inversions' settings and the update maxima, in one node).
+// Several inversions' settings in one launch: states st[0..count) and the conditions of the WHILE
+// nodes hs.h[0..nhandles); it also clears zero[0..nzero) (the SyN level graph begins every iteration
+// with it: its four inversions' settings, its two loops and the update maxima, in one node).
 struct InitHandles {
     cudaGraphConditionalHandle h[kMaxInitHandles];
 };
 __global__ void k_inv_init_many(InvState* __restrict__ st, int count, fw_invert_params prm,
-                                InitHandles hs, unsigned int* __restrict__ zero, int nzero) {
+                                InitHandles hs, int nhandles, unsigned int* __restrict__ zero,
+                                int nzero) {
     pdl_wait();
     const int i = threadIdx.x;
-    if (i < count) {
-        init_state(st + i, prm);
-        cudaGraphSetConditional(hs.h[i], st[i].go ? 1u : 0u);
-    }
+    if (i < count) init_state(st + i, prm);
+    if (i < nhandles) cudaGraphSetConditional(hs.h[i], prm.max_iterations > 0 ? 1u : 0u);
     if (i < nzero) zero[i] = 0u;
 }
 
@@ -438,6 +438,75 @@ __global__ void __launch_bounds__(256, 4) k_inv_fix(InvArgs a, float* __restrict
     fix_tiles(a, psi, res, st, defer, blockIdx.x, gridDim.x);
 }
 
+// ---- the same inversion of both sides of a SyN iteration, one launch of each kernel -----------
+//
+// The sides are independent (F and F^-1, M and M^-1), each with its own loop state st[2 * side],
+// partials, counter and deferred list, reduced in the single kernels' order. Twice the blocks a
+// launch and half the launches: on the coarse levels, where a launch is a few microseconds whatever
+// it does, the iteration's time follows the launches.
+struct InvPair {
+    InvArgs a;
+    const float* f[2];
+    float* psi[2];
+    float* res[2];
+    double* partials[2];
+    unsigned int* defer[2];
+    unsigned int* counter;  // [0, 1] the sides' step blocks, [2] the sides that are through
+    InvState* st;           // side s at st[2 * s]
+};
+
+__global__ void k_inv_init_pair(InvState* __restrict__ st, fw_invert_params prm) {
+    init_state(st + 2 * threadIdx.x, prm);
+}
+
+__global__ void __launch_bounds__(256) k_inv_bound_pair(const __grid_constant__ InvPair p, Lattice t) {
+    pdl_wait();
+    const int side = blockIdx.y;
+    InvState* st = p.st + 2 * side;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st->ndefer = 0u;
+        st->run = st->go;
+    }
+    if (!st->go) return;
+    bound_block(p.a, t, p.f[side], p.psi[side], st, blockIdx.x, gridDim.x);
+}
+
+__global__ void __launch_bounds__(256, FW_STEP_MIN_BLOCKS) k_inv_step_pair(
+    const __grid_constant__ InvPair p, int gx, cudaGraphConditionalHandle handle, int use_handle) {
+    pdl_wait();
+    const int side = (int)blockIdx.x >= gx ? 1 : 0;  // the first gx x blocks are side 0's
+    const int bx = (int)blockIdx.x - side * gx;
+    InvState* st = p.st + 2 * side;
+    if (!st->run) return;  // uniform over the side's blocks: the bound kernel set it
+    double sum = 0.0;
+    float mx = 0.0f;
+    step_block(p.a, bx, blockIdx.y, blockIdx.z, gx, p.f[side], p.psi[side], p.res[side], st,
+               p.defer[side], sum, mx);
+    const unsigned int bid = bx + gx * (blockIdx.y + gridDim.y * blockIdx.z);
+    reduce_and_finish(sum, mx, p.partials[side], p.counter + side, bid, gx * gridDim.y * gridDim.z,
+                      [&](double s, double m) {
+                          finish_step(st, s, m, (double)p.a.g.n);
+                          if (!use_handle) return;
+                          // the last side of the body sets the loop's condition
+                          __threadfence();
+                          const unsigned int sides = (unsigned int)(p.st[0].run + p.st[2].run);
+                          if (atomicAdd(p.counter + 2, 1u) == sides - 1u) {
+                              __threadfence();
+                              const int go = __ldcg(&p.st[0].go) | __ldcg(&p.st[2].go);
+                              cudaGraphSetConditional(handle, go ? 1u : 0u);
+                              p.counter[2] = 0u;
+                          }
+                      });
+}
+
+__global__ void __launch_bounds__(256, 4) k_inv_fix_pair(const __grid_constant__ InvPair p) {
+    pdl_wait();
+    const int side = blockIdx.y;
+    const InvState* st = p.st + 2 * side;
+    if (!st->run) return;  // an ended loop's deferred list has been applied
+    fix_tiles(p.a, p.psi[side], p.res[side], st, p.defer[side], blockIdx.x, gridDim.x);
+}
+
 // ---- batched inversions: every active subject of a batch, each with its own loop state ------
 //
 // Subject b's field, inverse and residual are at f / psi / res + b * stride, its partials at
@@ -584,14 +653,15 @@ int inversion_scratch(fw_ctx* ctx, const fw_field* field) {
 }
 
 int enqueue_inversion_inits(fw_ctx* ctx, InvState* st, int count, const fw_invert_params& prm,
-                            const cudaGraphConditionalHandle* handles, unsigned int* zero,
-                            int nzero) {
-    FW_CHECK(count >= 0 && count <= kMaxInitHandles && nzero >= 0 && nzero <= 32,
+                            const cudaGraphConditionalHandle* handles, int nhandles,
+                            unsigned int* zero, int nzero) {
+    FW_CHECK(count >= 0 && count <= 32 && nhandles >= 0 && nhandles <= kMaxInitHandles &&
+                 nzero >= 0 && nzero <= 32,
              "inversion inits: too many loops");
     InitHandles hs;
-    for (int i = 0; i < kMaxInitHandles; ++i) hs.h[i] = i < count ? handles[i] : 0;
+    for (int i = 0; i < kMaxInitHandles; ++i) hs.h[i] = i < nhandles ? handles[i] : 0;
     return launch_pdl(ctx, "k_inv_init_many", k_inv_init_many, dim3(1), dim3(32), 0, st, count,
-                      prm, hs, zero, nzero);
+                      prm, hs, nhandles, zero, nzero);
 }
 
 // One kernel of a body: 0 bound, 1 step, 2 fix (each returns at once when the loop has ended).
@@ -632,9 +702,50 @@ int enqueue_inversion_kernel(fw_ctx* ctx, const fw_field* field, fw_field* inver
     return launch_body_kernel(ctx, field, inverse, res, st, which, 0, 0);
 }
 
-size_t inv_scratch_doubles(const HostGrid& g) {
+// One inversion's scratch: its step's partials, then its deferred list (even, so that the next
+// one's partials stay aligned).
+static size_t inv_side_doubles(const HostGrid& g) {
     const size_t tiles = (size_t)inv_step_tiles(g), parts = (size_t)inv_step_parts(g);
-    return SLOT_PARTIALS + 2 * tiles + (parts + 1) / 2 + 16;
+    return (2 * tiles + (parts + 1) / 2 + 1) & ~(size_t)1;
+}
+
+size_t inv_scratch_doubles(const HostGrid& g) {
+    return SLOT_PARTIALS + 2 * inv_side_doubles(g) + 16;
+}
+
+int enqueue_inversion_pair_init(fw_ctx* ctx, const fw_invert_params& prm, InvState* st) {
+    k_inv_init_pair<<<1, 2, 0, ctx->stream>>>(st, prm);
+    return check_launch(ctx, "k_inv_init_pair");
+}
+
+int enqueue_inversion_pair_body(fw_ctx* ctx, const fw_field* const field[2],
+                                fw_field* const inverse[2], fw_field* const res[2], InvState* st,
+                                cudaGraphConditionalHandle handle, int use_handle) {
+    InvPair p;
+    p.a = inv_args(field[0], inverse[0]);
+    const dim3 g = step_grid(ctx, p.a);
+    const HostGrid& hg = field[0]->grid;
+    double* scratch = ctx->d_scratch + SLOT_PARTIALS;
+    for (int s = 0; s < 2; ++s) {
+        FW_CHECK(field[s]->ps == p.a.ps_f && inverse[s]->ps == p.a.ps_psi && res[s]->ps == p.a.ps_psi,
+                 "invert: the residual buffer does not match the inverse");
+        p.f[s] = field[s]->d;
+        p.psi[s] = inverse[s]->d;
+        p.res[s] = res[s]->d;
+        p.partials[s] = scratch + s * inv_side_doubles(hg);
+        p.defer[s] = reinterpret_cast<unsigned int*>(p.partials[s] + 2 * inv_step_tiles(hg));
+    }
+    p.counter = ctx->d_counter + 4;
+    p.st = st;
+    const Lattice t = lattice_of(p.a.g);
+    const unsigned int nb = (unsigned int)std::max<long long>(
+        1, std::min<long long>((t.count() + 255) / 256, 4LL * ctx->num_sms));
+    FW_TRY(launch_pdl(ctx, "k_inv_bound_pair", k_inv_bound_pair, dim3(nb, 2), dim3(256), 0, p, t));
+    FW_TRY(launch_pdl(ctx, "k_inv_step_pair", k_inv_step_pair, dim3(2 * g.x, g.y, g.z), dim3(256), 0,
+                      p, (int)g.x, handle, use_handle));
+    const unsigned int tiles = (unsigned int)inv_step_tiles(hg);
+    const unsigned int nf = std::max(1u, std::min(tiles, 2u * (unsigned int)ctx->num_sms));
+    return launch_pdl(ctx, "k_inv_fix_pair", k_inv_fix_pair, dim3(nf, 2), dim3(256), 0, p);
 }
 
 long long inv_bound_voxels(const HostGrid& g) {

@@ -146,7 +146,7 @@ int estimate(const fw_syn_request* q, uint64_t* out) {
     if (q->fixed == nullptr) b += 0;
     else b += 4 * C * (nf + nm);                       // uploaded inputs
     if (smooth) b += 4 * C * (nf + nm) + 24 * std::max(nf, nm);  // smoothed copies + Deriche temp
-    int fields = 4 + 2 + 1 /* inversion residual */ + (r->update_field_variance > 0 ? 2 : 0) +
+    int fields = 4 + 2 + 2 /* smoothing temporaries, inversion residuals */ +
                  (C > 1 ? 2 : 0) + (r->total_field_variance > 0 ? 1 : 0) + 2 /* outputs */;
     b += 12 * ps * (uint64_t)fields;
     b += 4 * (uint64_t)n * 2 * C;                      // warped images

@@ -306,6 +306,21 @@ __global__ void __launch_bounds__(XY_NT) k_smooth_xy(SmoothArgs a, const float* 
     smooth_xy_tile<R>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem_xy, in, tmp, ps_tmp);
 }
 
+// The xy pass of both sides of a SyN iteration in one launch: the first gx x blocks are side 0's.
+struct SmoothPair {
+    const float* in[2];
+    float* out[2];
+};
+template <int R>
+__global__ void __launch_bounds__(XY_NT) k_smooth_xy_pair(const __grid_constant__ SmoothArgs a,
+                                                          SmoothPair p, int gx) {
+    pdl_wait();
+    extern __shared__ __align__(16) float smem_xy[];
+    const int side = (int)blockIdx.x >= gx ? 1 : 0;
+    smooth_xy_tile<R>(a, (int)blockIdx.x - side * gx, blockIdx.y, blockIdx.z, smem_xy, p.in[side],
+                      p.out[side], a.ps_out);
+}
+
 // The xy pass of every active subject of a batch: input at in + b * stride (or at the subject's
 // multichannel accumulator), output into tmp + b * stride; tiles (x, y, slice) in the single
 // kernel's block order.
@@ -399,6 +414,19 @@ __global__ void __launch_bounds__(256, R <= 6 ? 3 : 2) k_smooth_z(SmoothArgs a, 
     }
 }
 
+// The z pass of both sides in one launch (the first gz x blocks are side 0's): tmp = p.in, and the
+// input that the blend reads is the output buffer itself; side s's max into max_bits[s].
+template <int R>
+__global__ void __launch_bounds__(256, R <= 6 ? 3 : 2) k_smooth_z_pair(
+    const __grid_constant__ SmoothArgs a, SmoothPair p, int gz, unsigned int* __restrict__ max_bits) {
+    pdl_wait();
+    const int side = (int)blockIdx.x >= gz ? 1 : 0;
+    float vmax = smooth_z_tile<R>(a, (int)blockIdx.x - side * gz, blockIdx.y, blockIdx.z, p.in[side],
+                                  a.ps_out, p.out[side], p.out[side], true);
+    vmax = warp_max_f(vmax);
+    if ((threadIdx.x & 31) == 0 && vmax > 0.0f) atomicMax(max_bits + side, __float_as_uint(vmax));
+}
+
 // The z pass of every active subject of a batch: tmp / in / out at + b * stride, the max of
 // subject b into max_bits[b * max_stride].
 template <int R>
@@ -435,6 +463,25 @@ int launch_smooth_xyz(fw_ctx* ctx, const SmoothArgs& a, const fw_field* in, fw_f
     dim3 g2((a.g.nz + Z_SEG - 1) / Z_SEG, (a.g.nx + 31) / 32, (a.g.ny + 7) / 8);
     return launch_pdl(ctx, "k_smooth_z", k_smooth_z<R>, g2, dim3(256), 0, a,
                       (const float*)tmp->d, (long long)tmp->ps, (const float*)in->d, out->d,
+                      d_max_bits);
+}
+
+// Both fields a[s] smoothed in place through tmp[s].
+template <int R>
+int launch_smooth_pair_r(fw_ctx* ctx, const SmoothArgs& a, fw_field* const f[2],
+                         fw_field* const tmp[2], unsigned int* d_max_bits) {
+    constexpr int HY = XY_T + 2 * R, HXP = (XY_T + 2 * R + 3) & ~3, NV = (4 + 2 * R + 3) / 4;
+    constexpr size_t bytes = sizeof(float) * (3 * HY * HXP + 4 * NV + 3 * HY * XY_T);
+    FW_CUDA(cudaFuncSetAttribute(k_smooth_xy_pair<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)bytes));
+    const SmoothPair xy{{f[0]->d, f[1]->d}, {tmp[0]->d, tmp[1]->d}};
+    const SmoothPair z{{tmp[0]->d, tmp[1]->d}, {f[0]->d, f[1]->d}};
+    const int gx = (a.g.nx + XY_T - 1) / XY_T, gz = (a.g.nz + Z_SEG - 1) / Z_SEG;
+    dim3 g1(2 * gx, (a.g.ny + XY_T - 1) / XY_T, a.g.nz);
+    FW_TRY(launch_pdl(ctx, "k_smooth_xy_pair", k_smooth_xy_pair<R>, g1, dim3(XY_NT), bytes, a, xy,
+                      gx));
+    dim3 g2(2 * gz, (a.g.nx + 31) / 32, (a.g.ny + 7) / 8);
+    return launch_pdl(ctx, "k_smooth_z_pair", k_smooth_z_pair<R>, g2, dim3(256), 0, a, z, gz,
                       d_max_bits);
 }
 
@@ -612,16 +659,16 @@ __global__ void k_f64_to_f32(const double* __restrict__ a, float* __restrict__ b
 
 }  // namespace
 
-int launch_smooth(fw_ctx* ctx, const fw_field* in, fw_field* out, double variance,
-                  unsigned int* d_max_bits, fw_field* tmp) {
-    SmoothArgs a;
+// The taps and blend of a smoothing on `g`; *same: the three axes have the same taps.
+static int smooth_args(const HostGrid& g, long long ps_in, long long ps_out, double variance,
+                       SmoothArgs& a, bool* same) {
     std::memset(&a, 0, sizeof(a));
-    a.g = dev_grid(in->grid);
-    a.ps_in = in->ps;
-    a.ps_out = out->ps;
+    a.g = dev_grid(g);
+    a.ps_in = ps_in;
+    a.ps_out = ps_out;
     int r[3];
     for (int ax = 0; ax < 3; ++ax) {
-        std::vector<double> k = gaussian_taps(variance, 0.001, in->grid.n[ax]);
+        std::vector<double> k = gaussian_taps(variance, 0.001, g.n[ax]);
         int rad = (int)k.size() / 2;
         if (rad > (MAX_TAPS - 1) / 2)
             return fail(FW_ERR_INVALID, "smooth field: the Gaussian kernel radius exceeds 24 voxels");
@@ -635,9 +682,49 @@ int launch_smooth(fw_ctx* ctx, const fw_field* in, fw_field* out, double varianc
     double w1 = variance < 0.5 ? 1.0 - variance / 0.5 : 1.0;
     a.w1 = (float)w1;
     a.w2 = (float)(1.0 - w1);
-    bool same = tmp != nullptr && r[0] == r[1] && r[1] == r[2];
-    for (int t = 0; same && t <= 2 * r[0]; ++t)
-        same = a.tx_[t] == a.ty_[t] && a.ty_[t] == a.tz_[t];
+    *same = r[0] == r[1] && r[1] == r[2];
+    for (int t = 0; *same && t <= 2 * r[0]; ++t)
+        *same = a.tx_[t] == a.ty_[t] && a.ty_[t] == a.tz_[t];
+    return 0;
+}
+
+int launch_smooth_pair(fw_ctx* ctx, fw_field* const f[2], fw_field* const tmp[2], double variance,
+                       unsigned int* d_max_bits, bool* in_tmp) {
+    SmoothArgs a;
+    bool same = false;
+    FW_TRY(smooth_args(f[0]->grid, f[0]->ps, f[0]->ps, variance, a, &same));
+    *in_tmp = false;
+    if (same) {
+        switch (a.rx) {
+            case 1: return launch_smooth_pair_r<1>(ctx, a, f, tmp, d_max_bits);
+            case 2: return launch_smooth_pair_r<2>(ctx, a, f, tmp, d_max_bits);
+            case 3: return launch_smooth_pair_r<3>(ctx, a, f, tmp, d_max_bits);
+            case 4: return launch_smooth_pair_r<4>(ctx, a, f, tmp, d_max_bits);
+            case 5: return launch_smooth_pair_r<5>(ctx, a, f, tmp, d_max_bits);
+            case 6: return launch_smooth_pair_r<6>(ctx, a, f, tmp, d_max_bits);
+            case 7: return launch_smooth_pair_r<7>(ctx, a, f, tmp, d_max_bits);
+            case 8: return launch_smooth_pair_r<8>(ctx, a, f, tmp, d_max_bits);
+            case 9: return launch_smooth_pair_r<9>(ctx, a, f, tmp, d_max_bits);
+            case 10: return launch_smooth_pair_r<10>(ctx, a, f, tmp, d_max_bits);
+            case 11: return launch_smooth_pair_r<11>(ctx, a, f, tmp, d_max_bits);
+            case 12: return launch_smooth_pair_r<12>(ctx, a, f, tmp, d_max_bits);
+            default: break;
+        }
+    }
+    // axes of different taps (an axis shorter than the kernel), wide kernels
+    for (int s = 0; s < 2; ++s)
+        FW_TRY(launch_smooth(ctx, f[s], tmp[s], variance, d_max_bits + s, nullptr));
+    *in_tmp = true;
+    return 0;
+}
+
+int launch_smooth(fw_ctx* ctx, const fw_field* in, fw_field* out, double variance,
+                  unsigned int* d_max_bits, fw_field* tmp) {
+    SmoothArgs a;
+    bool same = false;
+    FW_TRY(smooth_args(in->grid, in->ps, out->ps, variance, a, &same));
+    const int r[3] = {a.rx, a.ry, a.rz};
+    same = same && tmp != nullptr;
     if (same) {
         FW_CHECK(tmp->grid.same(in->grid) && tmp != in && tmp != out,
                  "smooth field: the temporary field must be a third field on the same grid");

@@ -10,13 +10,12 @@
 //
 // Graph design: every buffer of a level is allocated once, so the kernel sequence of an
 // iteration is the same every time. The whole level is captured as ONE CUDA graph: an outer
-// WHILE node whose body is the iteration, with each of the four inversions an inner WHILE node
-// whose condition the inversion step's last block sets (no host read-back inside the loop); the
-// iteration's first kernel sets the four loops' states and conditions and clears the update
-// maxima. A
-// single-thread record kernel at the end of the body runs the convergence monitor on the device,
-// writes the iteration record and sets the outer condition. The host launches one graph and
-// reads the records back once per level.
+// WHILE node whose body is the iteration, with each of the two inversions of both sides an inner
+// WHILE node whose condition the inversion step's last block sets (no host read-back inside the
+// loop); the iteration's first kernel sets the loops' states and conditions and clears the update
+// maxima. The two sides (F and M) share every launch. A record kernel at the end of the body runs
+// the convergence monitor on the device, writes the iteration record and sets the outer condition.
+// The host launches one graph and reads the records back once per level.
 #include <cuda_runtime.h>
 
 #include <cfloat>
@@ -42,14 +41,34 @@ __global__ void k_syn_level_init(SynDev* s, int level, int limit,
     if (use_handle) cudaGraphSetConditional(handle, run ? 1u : 0u);
 }
 
-__global__ void k_syn_record(SynDev* s, const double* __restrict__ cc,
-                             const unsigned int* __restrict__ max_bits,
-                             const InvState* __restrict__ inv, fw_syn_iteration* trace,
-                             int trace_cap, const volatile int* cancel,
-                             cudaGraphConditionalHandle handle, int use_handle) {
+// The end of an iteration. One thread does the work; the block first brings the state and the
+// scalars to shared memory in one step, because a thread that walks them in global memory waits for
+// them one after another (8.3 us a launch at any grid, @REC@).
+constexpr int RECORD_THREADS = 128;
+__global__ void __launch_bounds__(RECORD_THREADS) k_syn_record(
+    SynDev* s, const double* __restrict__ cc, const unsigned int* __restrict__ max_bits,
+    const InvState* __restrict__ inv, fw_syn_iteration* trace, int trace_cap,
+    const volatile int* cancel, cudaGraphConditionalHandle handle, int use_handle) {
     pdl_wait();
-    const int more = syn_record_step(s, cc, max_bits, inv, trace, trace_cap, cancel);
-    if (use_handle) cudaGraphSetConditional(handle, more ? 1u : 0u);
+    __shared__ SynDev ss;
+    __shared__ double scc[FW_MAX_CHANNELS * CC_STRIDE];
+    __shared__ InvState sinv[4];
+    static_assert(sizeof(SynDev) % 8 == 0 && sizeof(InvState) % 8 == 0, "copied in doubles");
+    const int t = threadIdx.x;
+    for (int i = t; i < (int)(sizeof(SynDev) / 8); i += RECORD_THREADS)
+        reinterpret_cast<double*>(&ss)[i] = reinterpret_cast<const double*>(s)[i];
+    for (int i = t; i < FW_MAX_CHANNELS * CC_STRIDE; i += RECORD_THREADS) scc[i] = cc[i];
+    for (int i = t; i < (int)(sizeof(sinv) / 8); i += RECORD_THREADS)
+        reinterpret_cast<double*>(sinv)[i] = reinterpret_cast<const double*>(inv)[i];
+    const unsigned int mb[2] = {max_bits[0], max_bits[1]};
+    __syncthreads();
+    if (t == 0) {
+        const int more = syn_record_step(&ss, scc, mb, sinv, trace, trace_cap, cancel);
+        if (use_handle) cudaGraphSetConditional(handle, more ? 1u : 0u);
+    }
+    __syncthreads();
+    for (int i = t; i < (int)(sizeof(SynDev) / 8); i += RECORD_THREADS)
+        reinterpret_cast<double*>(s)[i] = reinterpret_cast<const double*>(&ss)[i];
 }
 
 // acc += (w / |x|) x when |x| > eps (syn.rs:233-240), |x|^2 read from the device.
@@ -91,9 +110,10 @@ struct Level {
     std::vector<fw_image*> fmid, mmid;
     fw_field *dF = nullptr, *dM = nullptr;      // raw CC derivatives
     fw_field *accF = nullptr, *accM = nullptr;  // multichannel combination
-    fw_field *sF = nullptr, *sM = nullptr;      // smoothed updates
+    // the smoothings' temporaries, then the inversions' residuals of the last measurement
+    fw_field *sF = nullptr, *sM = nullptr;
     fw_field* T = nullptr;                      // total-field smoothing
-    fw_field* R = nullptr;                      // inversion residual of the last measurement
+    fw_field *uF = nullptr, *uM = nullptr;      // where the iteration left its updates (not owned)
     const fw_image* fmask = nullptr;            // recipe masks on their own grids (or none)
     const fw_image* mmask = nullptr;
     fw_image* fvalid = nullptr;                 // each given mask resolved on the level grid
@@ -114,9 +134,9 @@ void free_level_work(Level& L) {
     L.valid = L.fvalid = L.mvalid = nullptr;
     dense_mi_free(L.mi);
     L.mi = nullptr;
-    fw_field* fs[] = {L.dF, L.dM, L.accF, L.accM, L.sF, L.sM, L.T, L.R};
+    fw_field* fs[] = {L.dF, L.dM, L.accF, L.accM, L.sF, L.sM, L.T};
     for (auto* f : fs) fw_field_free(f);
-    L.dF = L.dM = L.accF = L.accM = L.sF = L.sM = L.T = L.R = nullptr;
+    L.dF = L.dM = L.accF = L.accM = L.sF = L.sM = L.T = L.uF = L.uM = nullptr;
 }
 
 int alloc_level_work(fw_ctx* ctx, const fw_syn_recipe* r, Level& L) {
@@ -129,14 +149,11 @@ int alloc_level_work(fw_ctx* ctx, const fw_syn_recipe* r, Level& L) {
     }
     FW_TRY(new_field(ctx, L.grid, &L.dF));
     FW_TRY(new_field(ctx, L.grid, &L.dM));
-    FW_TRY(new_field(ctx, L.grid, &L.R));
+    FW_TRY(new_field(ctx, L.grid, &L.sF));
+    FW_TRY(new_field(ctx, L.grid, &L.sM));
     if (L.channels > 1) {
         FW_TRY(new_field(ctx, L.grid, &L.accF));
         FW_TRY(new_field(ctx, L.grid, &L.accM));
-    }
-    if (r->update_field_variance > 0.0) {
-        FW_TRY(new_field(ctx, L.grid, &L.sF));
-        FW_TRY(new_field(ctx, L.grid, &L.sM));
     }
     if (r->total_field_variance > 0.0) FW_TRY(new_field(ctx, L.grid, &L.T));
     if (L.fmask) FW_TRY(new_image(ctx, L.grid, &L.fvalid));
@@ -153,7 +170,7 @@ struct RunDev {
     SynDev* syn;
     double* cc;              // [channels][CC_STRIDE]
     unsigned int* max_bits;  // [2]
-    InvState* inv;           // [4]
+    InvState* inv;           // [4]: F's two inversions, M's two
     fw_syn_iteration* trace;
     int trace_cap;
 };
@@ -183,26 +200,25 @@ int add_while_node(cudaStream_t s, cudaGraphConditionalHandle handle, cudaGraph_
 
 namespace {
 
-// One inversion: in graph mode a WHILE node around the body kernels on `h` (the iteration's first
-// kernel set the loop's state and condition); in direct mode its init kernel and a host loop.
-int enqueue_invert(fw_ctx* ctx, bool graph, const fw_field* field, fw_field* inverse,
-                   fw_field* res, InvState* st, cudaGraphConditionalHandle h) {
+// The same inversion of both sides (st: side s's state at st[2 s]): in graph mode a WHILE node around
+// the body kernels on `h` (the iteration's first kernel set the loops' states and condition); in
+// direct mode their init kernel and a host loop.
+int enqueue_invert_pair(fw_ctx* ctx, bool graph, fw_field* const field[2], fw_field* const inverse[2],
+                        fw_field* const res[2], InvState* st, cudaGraphConditionalHandle h) {
+    FW_TRY(inversion_scratch(ctx, field[0]));
     if (!graph) {
-        FW_TRY(enqueue_inversion_prefix(ctx, field, inverse, res, kSynInvert, st, 0, 0));
-        InvState hs;
+        FW_TRY(enqueue_inversion_pair_init(ctx, kSynInvert, st));
+        InvState hs[3];  // this inversion's states of both sides, the other inversion's between them
         for (int body = 0; body < kSynInvert.max_iterations; ++body) {
-            FW_TRY(enqueue_inversion_body(ctx, field, inverse, res, st, 0, 0));
-            FW_CUDA(cudaMemcpyAsync(ctx->h_pinned, st, sizeof(InvState), cudaMemcpyDeviceToHost,
+            FW_TRY(enqueue_inversion_pair_body(ctx, field, inverse, res, st, 0, 0));
+            FW_CUDA(cudaMemcpyAsync(ctx->h_pinned, st, sizeof(hs), cudaMemcpyDeviceToHost,
                                     ctx->stream));
             FW_TRY(sync(ctx));
-            std::memcpy(&hs, ctx->h_pinned, sizeof(hs));
-            if (!hs.go) break;
+            std::memcpy(hs, ctx->h_pinned, sizeof(hs));
+            if (!hs[0].go && !hs[2].go) break;
         }
         return 0;
     }
-    FW_CHECK(res->grid.same(inverse->grid) && res->ps == inverse->ps,
-             "invert: the residual buffer does not match the inverse");
-    FW_TRY(inversion_scratch(ctx, field));
     cudaStreamCaptureStatus status;
     cudaGraph_t g;
     const cudaGraphNode_t* deps;
@@ -222,7 +238,7 @@ int enqueue_invert(fw_ctx* ctx, bool graph, const fw_field* field, fw_field* inv
     FW_CUDA(cudaStreamBeginCaptureToGraph(ctx->aux, body, nullptr, nullptr, 0,
                                           cudaStreamCaptureModeRelaxed));
     ctx->stream = ctx->aux;
-    int rc = enqueue_inversion_body(ctx, field, inverse, res, st, h, 1);
+    int rc = enqueue_inversion_pair_body(ctx, field, inverse, res, st, h, 1);
     ctx->stream = main;
     cudaGraph_t out;
     cudaError_t e = cudaStreamEndCapture(ctx->aux, &out);
@@ -240,15 +256,15 @@ int enqueue_iteration(fw_ctx* ctx, bool graph, const fw_syn_recipe* r, Level& L,
                       const RunDev& d) {
     const int C = L.channels;
     // graph mode: one kernel begins the iteration -- the update maxima cleared, the four
-    // inversions' states and WHILE conditions set (their handles live in the graph being
-    // captured); direct mode: a memset, and each inversion's init kernel
-    cudaGraphConditionalHandle hinv[4] = {0, 0, 0, 0};
+    // inversions' states and their two WHILE conditions set (the handles live in the graph being
+    // captured); direct mode: a memset, and each pair of inversions' init kernel
+    cudaGraphConditionalHandle hinv[2] = {0, 0};
     if (graph) {
         cudaStreamCaptureStatus status;
         cudaGraph_t g;
         FW_CUDA(cudaStreamGetCaptureInfo(ctx->stream, &status, nullptr, &g, nullptr, nullptr));
         for (auto& h : hinv) FW_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, 0));
-        FW_TRY(enqueue_inversion_inits(ctx, d.inv, 4, kSynInvert, hinv, d.max_bits, 2));
+        FW_TRY(enqueue_inversion_inits(ctx, d.inv, 4, kSynInvert, hinv, 2, d.max_bits, 2));
     } else {
         FW_CUDA(cudaMemsetAsync(d.max_bits, 0, 2 * sizeof(unsigned int), ctx->stream));
     }
@@ -272,8 +288,16 @@ int enqueue_iteration(fw_ctx* ctx, bool graph, const fw_syn_recipe* r, Level& L,
         valid = L.valid;
     }
     for (int c = 0; c < C; ++c) {
-        FW_TRY(launch_warp(ctx, fs[c], L.Fi, nullptr, nullptr, L.fmid[c]->d, false, nullptr));
-        FW_TRY(launch_warp(ctx, ms[c], L.Mi, L.prior, initial, L.mmid[c]->d, false, nullptr));
+        if (L.prior) {
+            FW_TRY(launch_warp(ctx, fs[c], L.Fi, nullptr, nullptr, L.fmid[c]->d, false, nullptr));
+            FW_TRY(launch_warp(ctx, ms[c], L.Mi, L.prior, initial, L.mmid[c]->d, false, nullptr));
+        } else {
+            const fw_image* const src[2] = {fs[c], ms[c]};
+            const fw_field* const through[2] = {L.Fi, L.Mi};
+            const fw_affine* const affine[2] = {nullptr, initial};
+            float* const out[2] = {L.fmid[c]->d, L.mmid[c]->d};
+            FW_TRY(launch_warp_pair(ctx, src, through, affine, out));
+        }
         if (r->channel_metrics[c] == FW_METRIC_MATTES)
             FW_TRY(enqueue_dense_mi_pair(ctx, L.fmid[c], L.mmid[c], L.fvalid, L.mvalid, L.dF,
                                          L.dM, L.mi, d.cc + CC_STRIDE * c));
@@ -302,39 +326,36 @@ int enqueue_iteration(fw_ctx* ctx, bool graph, const fw_syn_recipe* r, Level& L,
         gF = L.accF;
         gM = L.accM;
     }
-    // update_total_field for both sides (syn.rs:422-445), one side after the other: smooth the
-    // update (variance in voxels^2) with its max |u/sp| fused; F <- F + (step / max) u(x + F) in
-    // place; optional total-field smoothing; the inversion pair. The sides only share scratch
-    // (the residual field R), so running them in turn gives the reference's fields.
-    struct Side {
-        fw_field* g;  // raw update (CC derivative or channel combination)
-        fw_field* s;  // smoothed update
-        fw_field* field;
-        fw_field* inverse;
-        unsigned int* max;
-        InvState* st;
-        const cudaGraphConditionalHandle* h;
-    } sides[2] = {{gF, L.sF, L.F, L.Fi, d.max_bits, d.inv, hinv},
-                  {gM, L.sM, L.M, L.Mi, d.max_bits + 1, d.inv + 2, hinv + 2}};
-    for (auto& s : sides) {
-        const fw_field* u = s.g;
-        if (r->update_field_variance > 0.0) {
-            FW_TRY(launch_smooth(ctx, s.g, s.s, r->update_field_variance, s.max, L.R));
-            u = s.s;
-        } else {
-            FW_TRY(launch_max_norm(ctx, s.g, s.max));
-        }
-        // compose in place: every voxel reads its own field value and the update elsewhere
-        FW_TRY(launch_compose(ctx, u, s.field, s.field, s.max, r->gradient_step));
-        if (r->total_field_variance > 0.0) {
-            FW_TRY(launch_smooth(ctx, s.field, L.T, r->total_field_variance, nullptr, L.R));
-            FW_CUDA(cudaMemcpyAsync(s.field->d, L.T->d, s.field->bytes, cudaMemcpyDeviceToDevice,
+    // update_total_field for both sides (syn.rs:422-445), each step one launch over the two, which
+    // share nothing: smooth the update (variance in voxels^2) with its max |u/sp| fused;
+    // F <- F + (step / max) u(x + F) in place; optional total-field smoothing; the inversion pair.
+    // 48 x 57 x 48 level of the 1 mm recipe: 0.2 ms an iteration one side after the other.
+    fw_field* u[2] = {gF, gM};
+    fw_field* work[2] = {L.sF, L.sM};
+    fw_field* field[2] = {L.F, L.M};
+    fw_field* inverse[2] = {L.Fi, L.Mi};
+    if (r->update_field_variance > 0.0) {
+        bool in_tmp = false;
+        FW_TRY(launch_smooth_pair(ctx, u, work, r->update_field_variance, d.max_bits, &in_tmp));
+        if (in_tmp)
+            for (int s = 0; s < 2; ++s) std::swap(u[s], work[s]);
+    } else {
+        for (int s = 0; s < 2; ++s) FW_TRY(launch_max_norm(ctx, u[s], d.max_bits + s));
+    }
+    L.uF = u[0];
+    L.uM = u[1];
+    // compose in place: every voxel reads its own field value and the update elsewhere
+    FW_TRY(launch_compose_pair(ctx, u, field, d.max_bits, r->gradient_step));
+    if (r->total_field_variance > 0.0) {
+        for (int s = 0; s < 2; ++s) {
+            FW_TRY(launch_smooth(ctx, field[s], L.T, r->total_field_variance, nullptr, work[s]));
+            FW_CUDA(cudaMemcpyAsync(field[s]->d, L.T->d, field[s]->bytes, cudaMemcpyDeviceToDevice,
                                     ctx->stream));
         }
-        // inverse = invert(field), then field = invert(inverse)
-        FW_TRY(enqueue_invert(ctx, graph, s.field, s.inverse, L.R, s.st, s.h[0]));
-        FW_TRY(enqueue_invert(ctx, graph, s.inverse, s.field, L.R, s.st + 1, s.h[1]));
     }
+    // inverse = invert(field), then field = invert(inverse)
+    FW_TRY(enqueue_invert_pair(ctx, graph, field, inverse, work, d.inv, hinv[0]));
+    FW_TRY(enqueue_invert_pair(ctx, graph, inverse, field, work, d.inv + 1, hinv[1]));
     return 0;
 }
 
@@ -517,7 +538,7 @@ int run_level_direct(fw_ctx* ctx, const fw_syn_recipe* r, Level& L,
     for (int it = 0; it < limit; ++it) {
         if (cancel_requested(ctx)) return fail(FW_ERR_CANCELLED, "registration cancelled");
         FW_TRY(enqueue_iteration(ctx, false, r, L, fs, ms, initial, d));
-        k_syn_record<<<1, 1, 0, ctx->stream>>>(d.syn, d.cc, d.max_bits, d.inv, trace_dev_base,
+        k_syn_record<<<1, RECORD_THREADS, 0, ctx->stream>>>(d.syn, d.cc, d.max_bits, d.inv, trace_dev_base,
                                               d.trace_cap, ctx->cancel_mapped_dev, 0, 0);
         FW_TRY(check_launch(ctx, "k_syn_record"));
         FW_CUDA(cudaMemcpyAsync(ctx->h_pinned, d.syn, sizeof(SynDev), cudaMemcpyDeviceToHost,
@@ -562,7 +583,7 @@ int run_level_graph(fw_ctx* ctx, const fw_syn_recipe* r, Level& L,
             if (!rc) {
                 // the context's cancel flag is read once per iteration: a cancel stops the
                 // level graph after the iteration in flight
-                rc = launch_pdl(ctx, "k_syn_record", k_syn_record, dim3(1), dim3(1), 0, d.syn,
+                rc = launch_pdl(ctx, "k_syn_record", k_syn_record, dim3(1), dim3(RECORD_THREADS), 0, d.syn,
                                 (const double*)d.cc, (const unsigned int*)d.max_bits,
                                 (const InvState*)d.inv, trace_dev_base, d.trace_cap,
                                 ctx->cancel_mapped_dev, h_it, 1);
@@ -605,9 +626,9 @@ int check_status(int status, bool masked) {
 }
 
 // Kernels per iteration outside the inversion bodies (for the launch counter).
-int kernels_per_iteration(const fw_syn_recipe* r, int mask_warps) {
-    int k = r->channels * 3 + (r->channels > 1 ? 2 * r->channels + 2 : 0) +
-            4 /*two-pass smoothing or max*/ + 2 /*compose*/ +
+int kernels_per_iteration(const fw_syn_recipe* r, int mask_warps, bool prior) {
+    int k = r->channels * (prior ? 3 : 2) + (r->channels > 1 ? 2 * r->channels + 2 : 0) +
+            2 /*two-pass smoothing or max*/ + 1 /*compose*/ +
             (r->total_field_variance > 0.0 ? 4 : 0) + 1 /*inversion inits*/ + 1 /*record*/ +
             mask_warps + (mask_warps == 2 ? 1 : 0) /*product*/;
     for (int c = 0; c < r->channels; ++c)
@@ -810,12 +831,15 @@ int syn_run_device(fw_ctx* ctx, const fw_syn_recipe* r, const fw_image* const* f
                 FW_CUDA(cudaMemcpy(all.data(), rs.d.trace, sizeof(fw_syn_iteration) * done,
                                    cudaMemcpyDeviceToHost));
             // the kernels the level graphs ran (direct launches are counted as they are made):
-            // every iteration's kernels, three per inversion body, one level init per level
+            // every iteration's kernels, three per inversion body of the two sides, one level init
+            // per level
             for (int q = 0; q < done && graphs; ++q) {
-                for (int s = 0; s < 4; ++s)
-                    ctx->stats.kernel_launches += 3 * (uint64_t)all[q].inversions[s].iterations;
-                ctx->stats.kernel_launches +=
-                    kernels_per_iteration(r, (fixed_mask ? 1 : 0) + (moving_mask ? 1 : 0));
+                for (int s = 0; s < 2; ++s)
+                    ctx->stats.kernel_launches +=
+                        3 * (uint64_t)std::max(all[q].inversions[s].iterations,
+                                               all[q].inversions[s + 2].iterations);
+                ctx->stats.kernel_launches += kernels_per_iteration(
+                    r, (fixed_mask ? 1 : 0) + (moving_mask ? 1 : 0), prior != nullptr);
             }
             if (graphs) ctx->stats.kernel_launches += (uint64_t)graph_levels;
             if (records && cap > 0)
@@ -939,7 +963,7 @@ int fw_syn_step_masked(fw_ctx* ctx, const fw_syn_recipe* recipe, const fw_image*
     }
     if (!rc) rc = enqueue_iteration(ctx, false, recipe, L, fs, ms, initial, rs.d);
     if (!rc) {
-        k_syn_record<<<1, 1, 0, ctx->stream>>>(rs.d.syn, rs.d.cc, rs.d.max_bits, rs.d.inv, rs.d.trace, 1,
+        k_syn_record<<<1, RECORD_THREADS, 0, ctx->stream>>>(rs.d.syn, rs.d.cc, rs.d.max_bits, rs.d.inv, rs.d.trace, 1,
                                               nullptr, 0, 0);
         rc = check_launch(ctx, "k_syn_record");
     }
@@ -947,8 +971,7 @@ int fw_syn_step_masked(fw_ctx* ctx, const fw_syn_recipe* recipe, const fw_image*
     for (int side = 0; side < 2 && !rc; ++side) {
         double* out = side == 0 ? fixed_update : moving_update;
         if (!out) continue;
-        fw_field* u = side == 0 ? (L.sF ? L.sF : (L.accF ? L.accF : L.dF))
-                                : (L.sM ? L.sM : (L.accM ? L.accM : L.dM));
+        fw_field* u = side == 0 ? L.uF : L.uM;
         rc = launch_scale_by_max(ctx, u, rs.d.max_bits + side, recipe->gradient_step);
         if (!rc) rc = fw_field_download(ctx, u, out);
     }

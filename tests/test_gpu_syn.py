@@ -77,6 +77,40 @@ def test_a_syn_step_from_a_deformed_state_matches(backend, pair):
     assert np.abs(mu - omu).max() <= 1e-4
 
 
+@pytest.mark.parametrize("size,variance,total", [((45, 37, 5), 3.0, 0.0), ((33, 9, 17), 0.0, 0.0),
+                                                 ((40, 30, 20), 0.3, 0.5), ((70, 21, 35), 3.0, 0.0)])
+def test_a_step_matches_on_every_route_of_its_two_sides(backend, size, variance, total):
+    """The sides' shared launches: an axis shorter than the kernel (taps that differ by axis), no
+    update smoothing, the blend below variance 0.5 with total-field smoothing, and tiles with
+    remainders; the fixed side starts from zero and the moving side deformed, so that their
+    inversions end at bodies of their own."""
+    from cases import image
+    case = dict(size=size, seed=41)
+    f, m = image(case), image(case, seed_offset=1)
+    r = SynRecipe(gradient_step=0.4, update_field_variance=variance, total_field_variance=total,
+                  cc_radius=2, iterations=[1], shrink_factors=[1], smoothing_sigmas=[0.0],
+                  convergence_threshold=-1.0)
+    og = O.make_grid(size)
+    from fastwarp_b200 import make_grid
+    g = make_grid(size)
+    shape = size[::-1] + (3,)
+    ostate = {k: np.zeros(shape) for k in ("f2m", "f2m_inv", "m2m", "m2m_inv")}
+    for _ in range(3):
+        O.syn_step(oracle_recipe(r), og, og, [f], og, [m], None, ostate)
+    for k in ("f2m", "f2m_inv"):
+        ostate[k] = np.zeros(shape)
+    ostate = {k: v.astype(np.float32).astype(np.float64) for k, v in ostate.items()}
+    state = {k: backend.upload_field(g, v) for k, v in ostate.items()}
+    fi, mi = (backend.upload_image(g, a.astype(np.float32)) for a in (f, m))
+    rec, fu, mu = syn_step(backend, r, [fi], [mi], None, state)
+    orec, ofu, omu = O.syn_step(oracle_recipe(r), og, og, [f], og, [m], None, ostate)
+    assert abs(rec["energy"] - orec.energy) <= 1e-5 * abs(orec.energy)
+    assert np.abs(fu - ofu).max() <= 1e-4 and np.abs(mu - omu).max() <= 1e-4
+    assert [s[0] for s in rec["inversions"]] == [s.iterations for s in orec.inversions]
+    for k in state:
+        assert np.abs(backend.download_field(state[k]) - ostate[k]).max() <= 1e-4
+
+
 def test_full_registration_matches_the_oracle(backend, pair):
     g, fixed, moving = pair
     r = config1(30)
