@@ -175,8 +175,8 @@ __global__ void k_inv_init(InvState* __restrict__ st, fw_invert_params prm,
     if (use_handle) cudaGraphSetConditional(handle, st->go ? 1u : 0u);
 }
 
-// Several inversions' settings in one launch: states st[0..count) and the conditions of the WHILE
-// nodes hs.h[0..nhandles); it also clears zero[0..nzero) (the SyN level graph begins every iteration
+// Several inversions' settings in one launch: states st[0..count), and the conditions of the WHILE
+// nodes hs.h[0..nhandles) cleared (the bodies ahead of a node set it); it also clears zero[0..nzero) (the SyN level graph begins every iteration
 // with it: its four inversions' settings, its two loops and the update maxima, in one node).
 struct InitHandles {
     cudaGraphConditionalHandle h[kMaxInitHandles];
@@ -187,7 +187,7 @@ __global__ void k_inv_init_many(InvState* __restrict__ st, int count, fw_invert_
     pdl_wait();
     const int i = threadIdx.x;
     if (i < count) init_state(st + i, prm);
-    if (i < nhandles) cudaGraphSetConditional(hs.h[i], prm.max_iterations > 0 ? 1u : 0u);
+    if (i < nhandles) cudaGraphSetConditional(hs.h[i], 0u);
     if (i < nzero) zero[i] = 0u;
 }
 

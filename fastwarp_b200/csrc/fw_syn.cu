@@ -43,7 +43,7 @@ __global__ void k_syn_level_init(SynDev* s, int level, int limit,
 
 // The end of an iteration. One thread does the work; the block first brings the state and the
 // scalars to shared memory in one step, because a thread that walks them in global memory waits for
-// them one after another (8.3 us a launch at any grid, @REC@).
+// them one after another (8.3 us a launch at any grid).
 constexpr int RECORD_THREADS = 128;
 __global__ void __launch_bounds__(RECORD_THREADS) k_syn_record(
     SynDev* s, const double* __restrict__ cc, const unsigned int* __restrict__ max_bits,
@@ -200,9 +200,16 @@ int add_while_node(cudaStream_t s, cudaGraphConditionalHandle handle, cudaGraph_
 
 namespace {
 
-// The same inversion of both sides (st: side s's state at st[2 s]): in graph mode a WHILE node around
-// the body kernels on `h` (the iteration's first kernel set the loops' states and condition); in
-// direct mode their init kernel and a host loop.
+// Bodies of an inversion that a level graph holds as plain nodes before the WHILE node of the rest.
+// A kernel of a body that does not run returns at once (about a microsecond, more for a big grid's
+// blocks), a WHILE node that runs takes about ten. Microseconds an iteration with no, one, two and
+// three plain bodies: 64^3 (2-3 bodies an inversion) 169, 164, 156, 153; 48 x 57 x 48 (one or two)
+// 124, 114, 116, 118; 96 x 114 x 96 361, 354, 356, 365; 193 x 229 x 193 1746, 1734, 1751, 1757.
+int plain_bodies(const HostGrid& g) { return g.count() < (1 << 19) ? 2 : 1; }
+
+// The same inversion of both sides (st: side s's state at st[2 s]): in graph mode the plain bodies
+// and a WHILE node around the body kernels on `h`, whose condition the iteration's first kernel
+// cleared and the last plain body's step sets; in direct mode an init kernel and a host loop.
 int enqueue_invert_pair(fw_ctx* ctx, bool graph, fw_field* const field[2], fw_field* const inverse[2],
                         fw_field* const res[2], InvState* st, cudaGraphConditionalHandle h) {
     FW_TRY(inversion_scratch(ctx, field[0]));
@@ -219,20 +226,11 @@ int enqueue_invert_pair(fw_ctx* ctx, bool graph, fw_field* const field[2], fw_fi
         }
         return 0;
     }
-    cudaStreamCaptureStatus status;
-    cudaGraph_t g;
-    const cudaGraphNode_t* deps;
-    size_t ndeps;
-    FW_CUDA(cudaStreamGetCaptureInfo(ctx->stream, &status, nullptr, &g, &deps, &ndeps));
-    cudaGraphNodeParams p = {cudaGraphNodeTypeConditional};
-    p.conditional.handle = h;
-    p.conditional.type = cudaGraphCondTypeWhile;
-    p.conditional.size = 1;
-    cudaGraphNode_t node;
-    FW_CUDA(cudaGraphAddNode(&node, g, deps, ndeps, &p));
-    cudaGraph_t body = p.conditional.phGraph_out[0];
-    FW_CUDA(cudaStreamUpdateCaptureDependencies(ctx->stream, &node, 1,
-                                                cudaStreamSetCaptureDependencies));
+    const int plain = plain_bodies(field[0]->grid);
+    for (int k = 0; k < plain; ++k)
+        FW_TRY(enqueue_inversion_pair_body(ctx, field, inverse, res, st, h, k == plain - 1));
+    cudaGraph_t body = nullptr;
+    FW_TRY(add_while_node(ctx->stream, h, &body));
     // capture the body on the auxiliary stream
     cudaStream_t main = ctx->stream;
     FW_CUDA(cudaStreamBeginCaptureToGraph(ctx->aux, body, nullptr, nullptr, 0,
