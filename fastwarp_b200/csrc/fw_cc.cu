@@ -909,6 +909,10 @@ static int cc_pair_common(fw_ctx* ctx, const fw_image* fixed, const fw_image* mo
         return fail(FW_ERR_INVALID, "cc metric: the images are not on one grid");
     if (valid && !valid->grid.same(fixed->grid))
         return fail(FW_ERR_INVALID, "cc metric: the mask is not on the virtual grid");
+    // the scratch grows before the result's place in it is taken (at most one block a column tile,
+    // or four waves of them: plan_launch)
+    const long long tiles = ((fixed->grid.n[0] + TX - 1) / TX) * ((fixed->grid.n[1] + CC_TY - 1) / CC_TY);
+    FW_TRY(ensure_scratch(ctx, SLOT_PARTIALS + 4 * (size_t)(tiles + 32LL * ctx->num_sms) + 16));
     fw_field *a = nullptr, *b = nullptr;
     FW_TRY(new_field(ctx, fixed->grid, &a));
     int rc = new_field(ctx, fixed->grid, &b);

@@ -815,6 +815,8 @@ int launch_inv_any(fw_ctx* ctx, const InvState* st, int st_stride, const BatchLi
 // Host-driven loop (Backend::invert): one read-back of the loop flag per body.
 int invert_field(fw_ctx* ctx, const fw_field* field, fw_field* inverse,
                  const fw_invert_params& prm, fw_invert_stats* stats) {
+    // the scratch grows before the state's place in it is taken
+    FW_TRY(inversion_scratch(ctx, field));
     InvState* st = reinterpret_cast<InvState*>(ctx->d_scratch + SLOT_INV);
     fw_field* res = nullptr;  // the residual of the last measurement
     FW_TRY(new_field(ctx, inverse->grid, &res));

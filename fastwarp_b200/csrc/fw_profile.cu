@@ -3,6 +3,8 @@
 // kernels of one SyN iteration at a given level grid).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include <cstring>
 
 #include "fw_internal.cuh"
@@ -49,7 +51,9 @@ int fw_time_kernels(fw_ctx* ctx, const fw_image* fixed, const fw_image* moving, 
     if (!rc) rc = fw_field_zero(ctx, &cg, &w);
     if (!rc) rc = fw_field_zero(ctx, &cg, &e);
     if (!rc) rc = new_image(ctx, g, &out);
-    if (!rc) rc = ensure_scratch(ctx, SLOT_PARTIALS + (size_t)(1 << 20));
+    if (!rc)  // before the slots' places in it are taken
+        rc = ensure_scratch(ctx, std::max<size_t>(SLOT_PARTIALS + (size_t)(1 << 20),
+                                                  inv_scratch_doubles(g)));
     Events ev;
     if (!rc && (cudaEventCreate(&ev.a) != cudaSuccess || cudaEventCreate(&ev.b) != cudaSuccess))
         rc = fail(FW_ERR_CUDA, "event creation failed");

@@ -455,3 +455,22 @@ def test_buffers_of_sizes_no_longer_used_go_back_to_the_pool(backend):
         e = b.zero_field(make_grid((422, 422, 422)))  # the kept buffer serves the same shape
         assert b.cached_bytes() == nbytes(322)
         e.free()
+
+
+def test_a_context_whose_first_call_is_a_large_inversion(backend):
+    """The scratch of a context grows with the grid: the loop's state must not be left in what it
+    was before (its results are those of a context that had grown already)."""
+    from fastwarp_b200 import CudaBackend
+    g = make_grid((205, 190, 201))
+    rng = np.random.default_rng(4)
+    u = np.zeros((201, 190, 205, 3))
+    u[40:160, 40:150, 40:160] = rng.uniform(-0.4, 0.4, 3)
+    out = []
+    for k in range(2):
+        with CudaBackend(0) as b:
+            if k == 1:
+                b.invert(b.upload_field(g, u), b.zero_field(g))
+            inv, stats = b.invert(b.upload_field(g, u), b.zero_field(g))
+            out.append((b.download_field(inv), stats))
+    assert out[0][1] == out[1][1]
+    assert np.array_equal(out[0][0], out[1][0])
