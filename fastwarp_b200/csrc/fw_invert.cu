@@ -825,19 +825,16 @@ int invert_field(fw_ctx* ctx, const fw_field* field, fw_field* inverse,
         ~Free() { fw_field_free(f); }
     } guard{res};
     FW_TRY(enqueue_inversion_prefix(ctx, field, inverse, res, prm, st, 0, 0));
-    InvState h;
-    for (int body = 0; body < std::max(prm.max_iterations, 0); ++body) {
+    InvState h{};
+    if (prm.max_iterations <= 0) FW_TRY(sync(ctx));
+    for (int body = 0; body < prm.max_iterations; ++body) {
         FW_TRY(enqueue_inversion_body(ctx, field, inverse, res, st, 0, 0));
         FW_CUDA(cudaMemcpyAsync(ctx->h_pinned, st, sizeof(InvState), cudaMemcpyDeviceToHost,
                                 ctx->stream));
-        FW_TRY(sync(ctx));
+        FW_TRY(sync(ctx));  // the state that ends the loop is the one it reports
         std::memcpy(&h, ctx->h_pinned, sizeof(h));
         if (!h.go) break;
     }
-    FW_CUDA(cudaMemcpyAsync(ctx->h_pinned, st, sizeof(InvState), cudaMemcpyDeviceToHost,
-                            ctx->stream));
-    FW_TRY(sync(ctx));
-    std::memcpy(&h, ctx->h_pinned, sizeof(h));
     stats->iterations = h.executed;
     stats->mean_error_norm = h.executed == 0 ? 0.0 : h.mean;
     stats->max_error_norm = h.executed == 0 ? 0.0 : h.max;
