@@ -679,7 +679,9 @@ __global__ void __launch_bounds__(CC_NT, CC_MIN_BLOCKS) k_cc_pair_batch(
 // Grid of a launch: TX x TY column tiles times z chunks. About three and a half waves of resident
 // CTAs (measured at the 193 x 229 x 193 finest level, r = 4: 8 chunks 0.398 ms, 5 chunks 0.401 ms,
 // 2 chunks -- less than one wave -- 0.426 ms), with chunks no thinner than 2R slices, the filling
-// steps every chunk pays before its first output.
+// steps every chunk pays before its first output -- except where that leaves resident slots empty (the
+// coarse levels), where chunks go down to 4 slices: an iteration at 48 x 57 x 48 takes 116 us with
+// chunks of 8, 110 with 4 or 3, 112 with 2.
 template <int R, int TY, bool MK, int MODE, class Acc = SumF64>
 int plan_launch(CcArgs& a, int num_sms, dim3* grid) {
     using L = Layout<R, TY, MK>;
@@ -697,6 +699,8 @@ int plan_launch(CcArgs& a, int num_sms, dim3* grid) {
     const long long slots = (long long)occ * num_sms;
     long long best = (7 * slots + tiles) / (2 * tiles);  // round(3.5 slots / tiles)
     best = std::min<long long>(best, a.g.nz / (2 * R));
+    if (best * tiles < slots)
+        best = std::max<long long>(best, std::min<long long>(slots / tiles, a.g.nz / 4));
     best = std::max<long long>(best, 1);
     a.zchunk = (int)((a.g.nz + best - 1) / best);
     g.z = (a.g.nz + a.zchunk - 1) / a.zchunk;
