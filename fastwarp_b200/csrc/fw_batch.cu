@@ -628,10 +628,12 @@ int setup_level(Run& run, BatchLevel& L, const BatchLevel* prev, const HostGrid&
             for (int s = 0; s < B; ++s) {
                 fw_field src = view(ctx, *prev, *old[q], s);
                 fw_field dst = view(ctx, L, *state[q], s);
+                const fw_field* from = &src;
+                fw_field* to = &dst;
                 if (prev->grid.same(lg))
                     FW_CUDA(cudaMemcpyAsync(dst.d, src.d, dst.bytes, cudaMemcpyDeviceToDevice, ctx->stream));
                 else
-                    FW_TRY(launch_resample(ctx, &src, &dst));
+                    FW_TRY(launch_resample(ctx, &from, &to, 1));
             }
     }
     Buf* work[5] = {&L.dF, &L.dM, &L.sF, &L.sM, &L.R};

@@ -752,18 +752,19 @@ int launch_image_product(fw_ctx* ctx, const fw_image* a, const fw_image* b, fw_i
 int launch_compose(fw_ctx* ctx, const fw_field* disp, const fw_field* warping, fw_field* out,
                    const unsigned int* d_scale_max_bits, double step);
 // The two sides of a SyN iteration in one launch each (fields of one grid and plane stride): the
-// plain warps; the smoothing of f[s] through tmp[s] with its max |u/sp| in d_max_bits[s] (the result
-// replaces f[s], or lies in tmp[s] when *in_tmp); the composition in place.
+// plain warps; the smoothing of one or two fields f[s] through tmp[s] with its max |u/sp| in
+// d_max_bits[s] (the result replaces f[s], or lies in tmp[s] when *in_tmp); the composition in place.
 int launch_warp_pair(fw_ctx* ctx, const fw_image* const src[2], const fw_field* const field[2],
                      const fw_affine* const affine[2], float* const out[2]);
-int launch_smooth_pair(fw_ctx* ctx, fw_field* const f[2], fw_field* const tmp[2], double variance,
-                       unsigned int* d_max_bits, bool* in_tmp);
+int launch_smooth_sides(fw_ctx* ctx, fw_field* const* f, fw_field* const* tmp, int sides,
+                        double variance, unsigned int* d_max_bits, bool* in_tmp);
 int launch_compose_pair(fw_ctx* ctx, const fw_field* const update[2], fw_field* const field[2],
                         const unsigned int* d_max_bits, double step);
 int launch_scale_by_max(fw_ctx* ctx, fw_field* f, const unsigned int* d_max_bits, double step);
 int invert_field(fw_ctx* ctx, const fw_field* field, fw_field* inverse,
                  const fw_invert_params& prm, fw_invert_stats* stats);
-int launch_resample(fw_ctx* ctx, const fw_field* f, fw_field* out);
+// f[0 .. count) (at most 4, of one grid) onto the grid of out[0 .. count).
+int launch_resample(fw_ctx* ctx, const fw_field* const* f, fw_field* const* out, int count);
 int launch_smooth_recursive(fw_ctx* ctx, const fw_image* img, const double sigma_mm[3],
                             fw_image* out);
 int reduce_l2(fw_ctx* ctx, const fw_field* f, double* d_out);

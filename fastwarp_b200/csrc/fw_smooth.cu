@@ -312,8 +312,7 @@ struct SmoothPair {
     float* out[2];
 };
 template <int R>
-__global__ void __launch_bounds__(XY_NT) k_smooth_xy_pair(const __grid_constant__ SmoothArgs a,
-                                                          SmoothPair p, int gx) {
+__global__ void __launch_bounds__(XY_NT) k_smooth_xy_pair(SmoothArgs a, SmoothPair p, int gx) {
     pdl_wait();
     extern __shared__ __align__(16) float smem_xy[];
     const int side = (int)blockIdx.x >= gx ? 1 : 0;
@@ -418,7 +417,7 @@ __global__ void __launch_bounds__(256, R <= 6 ? 3 : 2) k_smooth_z(SmoothArgs a, 
 // input that the blend reads is the output buffer itself; side s's max into max_bits[s].
 template <int R>
 __global__ void __launch_bounds__(256, R <= 6 ? 3 : 2) k_smooth_z_pair(
-    const __grid_constant__ SmoothArgs a, SmoothPair p, int gz, unsigned int* __restrict__ max_bits) {
+    SmoothArgs a, SmoothPair p, int gz, unsigned int* __restrict__ max_bits) {
     pdl_wait();
     const int side = (int)blockIdx.x >= gz ? 1 : 0;
     float vmax = smooth_z_tile<R>(a, (int)blockIdx.x - side * gz, blockIdx.y, blockIdx.z, p.in[side],
@@ -466,16 +465,21 @@ int launch_smooth_xyz(fw_ctx* ctx, const SmoothArgs& a, const fw_field* in, fw_f
                       d_max_bits);
 }
 
-// Both fields a[s] smoothed in place through tmp[s].
+// Both fields f[s] smoothed in place through tmp[s].
 template <int R>
-int launch_smooth_pair_r(fw_ctx* ctx, const SmoothArgs& a, fw_field* const f[2],
-                         fw_field* const tmp[2], unsigned int* d_max_bits) {
+int launch_smooth_sides_r(fw_ctx* ctx, const SmoothArgs& a, fw_field* const* f,
+                          fw_field* const* tmp, unsigned int* d_max_bits) {
     constexpr int HY = XY_T + 2 * R, HXP = (XY_T + 2 * R + 3) & ~3, NV = (4 + 2 * R + 3) / 4;
     constexpr size_t bytes = sizeof(float) * (3 * HY * HXP + 4 * NV + 3 * HY * XY_T);
     FW_CUDA(cudaFuncSetAttribute(k_smooth_xy_pair<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)bytes));
-    const SmoothPair xy{{f[0]->d, f[1]->d}, {tmp[0]->d, tmp[1]->d}};
-    const SmoothPair z{{tmp[0]->d, tmp[1]->d}, {f[0]->d, f[1]->d}};
+    SmoothPair xy{}, z{};
+    for (int s = 0; s < 2; ++s) {
+        xy.in[s] = f[s]->d;
+        xy.out[s] = tmp[s]->d;
+        z.in[s] = tmp[s]->d;
+        z.out[s] = f[s]->d;
+    }
     const int gx = (a.g.nx + XY_T - 1) / XY_T, gz = (a.g.nz + Z_SEG - 1) / Z_SEG;
     dim3 g1(2 * gx, (a.g.ny + XY_T - 1) / XY_T, a.g.nz);
     FW_TRY(launch_pdl(ctx, "k_smooth_xy_pair", k_smooth_xy_pair<R>, g1, dim3(XY_NT), bytes, a, xy,
@@ -557,9 +561,19 @@ int deriche_zero_order(double sigma, double spacing, Deriche& out) {
 
 // One thread per line along `axis` (pyramid.rs:240-300): the causal pass goes to `tmp`, the
 // anticausal pass walks back with its last four inputs and outputs in registers and writes
-// causal + anticausal to `out`. Lines of the y and z axes are coalesced across threads.
-__global__ void k_deriche(const double* __restrict__ in, double* __restrict__ tmp,
-                          double* __restrict__ out, int nx, int ny, int nz, int axis, Deriche c) {
+// causal + anticausal to `out`. Lines of the y and z axes are coalesced across threads. The first
+// axis reads the float32 image and the last writes one (In, Out), in float64 between.
+//
+// A line is a serial chain, and a grid of lines is about ten warps an SM: what bounds it is the
+// latency of its loads, so they are taken DERICHE_BATCH at a time, the next batch in flight while
+// one is worked on. An image of 193 x 229 x 193 takes 275 us (z 57, x 152 for its uncoalesced lines,
+// y 66; 600 with one load at a time and the conversions as passes of their own).
+constexpr int DERICHE_BATCH = 8;
+template <class In, class Out>
+__global__ void __launch_bounds__(64) k_deriche(const In* __restrict__ in, double* __restrict__ tmp,
+                                                Out* __restrict__ out, int nx, int ny, int nz,
+                                                int axis, const __grid_constant__ Deriche c) {
+    constexpr int B = DERICHE_BATCH;
     long long line = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long base, stride;
     int ln;
@@ -581,10 +595,10 @@ __global__ void k_deriche(const double* __restrict__ in, double* __restrict__ tm
         ln = nz;
     }
     const double *n = c.n, *d = c.d, *m = c.m, *bn = c.bn, *bm = c.bm;
-    const double* x = in + base;
+    const In* x = in + base;
     double* ca = tmp + base;
-    double* o = out + base;
-#define X(i) x[(long long)(i) * stride]
+    Out* o = out + base;
+    auto X = [&](int i) { return (double)x[(long long)i * stride]; };
     double v1 = X(0);
     double c0 = X(0) * n[0] + v1 * n[1] + v1 * n[2] + v1 * n[3];
     double c1 = X(1) * n[0] + v1 * n[1] + v1 * n[2] + v1 * n[3];
@@ -601,18 +615,32 @@ __global__ void k_deriche(const double* __restrict__ in, double* __restrict__ tm
     {
         double xm1 = X(3), xm2 = X(2), xm3 = X(1);
         double cm1 = c3, cm2 = c2, cm3 = c1, cm4 = c0;
-        for (int i = 4; i < ln; ++i) {
-            double xi = X(i);
-            double ci = xi * n[0] + xm1 * n[1] + xm2 * n[2] + xm3 * n[3];
-            ci -= cm1 * d[0] + cm2 * d[1] + cm3 * d[2] + cm4 * d[3];
-            ca[(long long)i * stride] = ci;
-            xm3 = xm2;
-            xm2 = xm1;
-            xm1 = xi;
-            cm4 = cm3;
-            cm3 = cm2;
-            cm2 = cm1;
-            cm1 = ci;
+        In cur[B], nxt[B];
+        auto load = [&](int i, In b[B]) {  // inputs i .. i + B - 1 (past the end: unused)
+#pragma unroll
+            for (int t = 0; t < B; ++t)
+                if (i + t < ln) b[t] = x[(long long)(i + t) * stride];
+        };
+        load(4, cur);
+        for (int i = 4; i < ln; i += B) {
+            load(i + B, nxt);
+#pragma unroll
+            for (int t = 0; t < B; ++t) {
+                if (i + t >= ln) break;
+                const double xi = (double)cur[t];
+                double ci = xi * n[0] + xm1 * n[1] + xm2 * n[2] + xm3 * n[3];
+                ci -= cm1 * d[0] + cm2 * d[1] + cm3 * d[2] + cm4 * d[3];
+                ca[(long long)(i + t) * stride] = ci;
+                xm3 = xm2;
+                xm2 = xm1;
+                xm1 = xi;
+                cm4 = cm3;
+                cm3 = cm2;
+                cm2 = cm1;
+                cm1 = ci;
+            }
+#pragma unroll
+            for (int t = 0; t < B; ++t) cur[t] = nxt[t];
         }
     }
     double v2 = X(ln - 1);
@@ -624,37 +652,47 @@ __global__ void k_deriche(const double* __restrict__ in, double* __restrict__ tm
     e2 -= e1 * d[0] + v2 * bm[1] + v2 * bm[2] + v2 * bm[3];
     e3 -= e2 * d[0] + e1 * d[1] + v2 * bm[2] + v2 * bm[3];
     e4 -= e3 * d[0] + e2 * d[1] + e1 * d[2] + v2 * bm[3];
-    o[(long long)(ln - 1) * stride] = ca[(long long)(ln - 1) * stride] + e1;
-    o[(long long)(ln - 2) * stride] = ca[(long long)(ln - 2) * stride] + e2;
-    o[(long long)(ln - 3) * stride] = ca[(long long)(ln - 3) * stride] + e3;
-    o[(long long)(ln - 4) * stride] = ca[(long long)(ln - 4) * stride] + e4;
+    o[(long long)(ln - 1) * stride] = (Out)(ca[(long long)(ln - 1) * stride] + e1);
+    o[(long long)(ln - 2) * stride] = (Out)(ca[(long long)(ln - 2) * stride] + e2);
+    o[(long long)(ln - 3) * stride] = (Out)(ca[(long long)(ln - 3) * stride] + e3);
+    o[(long long)(ln - 4) * stride] = (Out)(ca[(long long)(ln - 4) * stride] + e4);
     // an[i-1] = x[i] m0 + x[i+1] m1 + x[i+2] m2 + x[i+3] m3 - (an[i] d0 + an[i+1] d1 + an[i+2] d2 + an[i+3] d3)
     double xp1 = X(ln - 3), xp2 = X(ln - 2), xp3 = X(ln - 1);  // x[i+1..i+3] at i = ln - 4
     double a0 = e4, a1 = e3, a2 = e2, a3 = e1;                 // an[i..i+3] at i = ln - 4
-    for (int i = ln - 4; i >= 1; --i) {
-        double xi = X(i);
-        double an = xi * m[0] + xp1 * m[1] + xp2 * m[2] + xp3 * m[3];
-        an -= a0 * d[0] + a1 * d[1] + a2 * d[2] + a3 * d[3];
-        o[(long long)(i - 1) * stride] = ca[(long long)(i - 1) * stride] + an;
-        xp3 = xp2;
-        xp2 = xp1;
-        xp1 = xi;
-        a3 = a2;
-        a2 = a1;
-        a1 = a0;
-        a0 = an;
+    In cur[B], nxt[B];
+    double kc[B], kn[B];
+    auto load = [&](int i, In b[B], double k[B]) {  // inputs i, i - 1, ... and causal values one below
+#pragma unroll
+        for (int t = 0; t < B; ++t)
+            if (i - t >= 1) {
+                b[t] = x[(long long)(i - t) * stride];
+                k[t] = ca[(long long)(i - t - 1) * stride];
+            }
+    };
+    load(ln - 4, cur, kc);
+    for (int i = ln - 4; i >= 1; i -= B) {
+        load(i - B, nxt, kn);
+#pragma unroll
+        for (int t = 0; t < B; ++t) {
+            if (i - t < 1) break;
+            const double xi = (double)cur[t];
+            double an = xi * m[0] + xp1 * m[1] + xp2 * m[2] + xp3 * m[3];
+            an -= a0 * d[0] + a1 * d[1] + a2 * d[2] + a3 * d[3];
+            o[(long long)(i - t - 1) * stride] = (Out)(kc[t] + an);
+            xp3 = xp2;
+            xp2 = xp1;
+            xp1 = xi;
+            a3 = a2;
+            a2 = a1;
+            a1 = a0;
+            a0 = an;
+        }
+#pragma unroll
+        for (int t = 0; t < B; ++t) {
+            cur[t] = nxt[t];
+            kc[t] = kn[t];
+        }
     }
-#undef X
-}
-
-__global__ void k_f32_to_f64(const float* __restrict__ a, double* __restrict__ b, long long n) {
-    long long l = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (l < n) b[l] = a[l];
-}
-
-__global__ void k_f64_to_f32(const double* __restrict__ a, float* __restrict__ b, long long n) {
-    long long l = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (l < n) b[l] = (float)a[l];
 }
 
 }  // namespace
@@ -688,31 +726,33 @@ static int smooth_args(const HostGrid& g, long long ps_in, long long ps_out, dou
     return 0;
 }
 
-int launch_smooth_pair(fw_ctx* ctx, fw_field* const f[2], fw_field* const tmp[2], double variance,
-                       unsigned int* d_max_bits, bool* in_tmp) {
+int launch_smooth_sides(fw_ctx* ctx, fw_field* const* f, fw_field* const* tmp, int sides,
+                        double variance, unsigned int* d_max_bits, bool* in_tmp) {
     SmoothArgs a;
     bool same = false;
     FW_TRY(smooth_args(f[0]->grid, f[0]->ps, f[0]->ps, variance, a, &same));
     *in_tmp = false;
+    if (same && sides == 1 && a.rx <= 12)
+        return launch_smooth(ctx, f[0], f[0], variance, d_max_bits, tmp[0]);
     if (same) {
         switch (a.rx) {
-            case 1: return launch_smooth_pair_r<1>(ctx, a, f, tmp, d_max_bits);
-            case 2: return launch_smooth_pair_r<2>(ctx, a, f, tmp, d_max_bits);
-            case 3: return launch_smooth_pair_r<3>(ctx, a, f, tmp, d_max_bits);
-            case 4: return launch_smooth_pair_r<4>(ctx, a, f, tmp, d_max_bits);
-            case 5: return launch_smooth_pair_r<5>(ctx, a, f, tmp, d_max_bits);
-            case 6: return launch_smooth_pair_r<6>(ctx, a, f, tmp, d_max_bits);
-            case 7: return launch_smooth_pair_r<7>(ctx, a, f, tmp, d_max_bits);
-            case 8: return launch_smooth_pair_r<8>(ctx, a, f, tmp, d_max_bits);
-            case 9: return launch_smooth_pair_r<9>(ctx, a, f, tmp, d_max_bits);
-            case 10: return launch_smooth_pair_r<10>(ctx, a, f, tmp, d_max_bits);
-            case 11: return launch_smooth_pair_r<11>(ctx, a, f, tmp, d_max_bits);
-            case 12: return launch_smooth_pair_r<12>(ctx, a, f, tmp, d_max_bits);
+            case 1: return launch_smooth_sides_r<1>(ctx, a, f, tmp, d_max_bits);
+            case 2: return launch_smooth_sides_r<2>(ctx, a, f, tmp, d_max_bits);
+            case 3: return launch_smooth_sides_r<3>(ctx, a, f, tmp, d_max_bits);
+            case 4: return launch_smooth_sides_r<4>(ctx, a, f, tmp, d_max_bits);
+            case 5: return launch_smooth_sides_r<5>(ctx, a, f, tmp, d_max_bits);
+            case 6: return launch_smooth_sides_r<6>(ctx, a, f, tmp, d_max_bits);
+            case 7: return launch_smooth_sides_r<7>(ctx, a, f, tmp, d_max_bits);
+            case 8: return launch_smooth_sides_r<8>(ctx, a, f, tmp, d_max_bits);
+            case 9: return launch_smooth_sides_r<9>(ctx, a, f, tmp, d_max_bits);
+            case 10: return launch_smooth_sides_r<10>(ctx, a, f, tmp, d_max_bits);
+            case 11: return launch_smooth_sides_r<11>(ctx, a, f, tmp, d_max_bits);
+            case 12: return launch_smooth_sides_r<12>(ctx, a, f, tmp, d_max_bits);
             default: break;
         }
     }
     // axes of different taps (an axis shorter than the kernel), wide kernels
-    for (int s = 0; s < 2; ++s)
+    for (int s = 0; s < sides; ++s)
         FW_TRY(launch_smooth(ctx, f[s], tmp[s], variance, d_max_bits + s, nullptr));
     *in_tmp = true;
     return 0;
@@ -816,37 +856,32 @@ int launch_smooth_recursive(fw_ctx* ctx, const fw_image* img, const double sigma
         if (g.n[ax] < 4) return fail(FW_ERR_INVALID, "smoothing: an axis has fewer than 4 voxels");
         if (!(sigma_mm[ax] > 0.0)) return fail(FW_ERR_INVALID, "smoothing: sigma must be greater than zero");
     }
-    double *vol = nullptr, *tmp = nullptr, *nxt = nullptr;
-    FW_TRY(dev_alloc(ctx, sizeof(double) * n, (void**)&vol));
-    int rc = dev_alloc(ctx, sizeof(double) * n, (void**)&tmp);
-    if (!rc) rc = dev_alloc(ctx, sizeof(double) * n, (void**)&nxt);
-    if (rc) {
-        dev_free(ctx, vol, sizeof(double) * n);
-        dev_free(ctx, tmp, sizeof(double) * n);
-        return rc;
-    }
-    unsigned int blocks = (unsigned int)((n + 255) / 256);
-    k_f32_to_f64<<<blocks, 256, 0, ctx->stream>>>(img->d, vol, n);
-    rc = check_launch(ctx, "k_f32_to_f64");
-    const int order[3] = {2, 0, 1};  // SmoothingRecursiveGaussianImageFilter: z, x, y
-    for (int oi = 0; oi < 3 && !rc; ++oi) {
-        int ax = order[oi];
-        Deriche c;
-        rc = deriche_zero_order(sigma_mm[ax], g.sp[ax], c);
-        if (rc) break;
-        long long lines = n / g.n[ax];
-        k_deriche<<<(unsigned int)((lines + 127) / 128), 128, 0, ctx->stream>>>(
-            vol, tmp, nxt, (int)g.n[0], (int)g.n[1], (int)g.n[2], ax, c);
-        rc = check_launch(ctx, "k_deriche");
-        std::swap(vol, nxt);
-    }
+    // SmoothingRecursiveGaussianImageFilter: z, x, y
+    double *tmp = nullptr, *z = nullptr, *x = nullptr;
+    FW_TRY(dev_alloc(ctx, sizeof(double) * n, (void**)&tmp));
+    int rc = dev_alloc(ctx, sizeof(double) * n, (void**)&z);
+    if (!rc) rc = dev_alloc(ctx, sizeof(double) * n, (void**)&x);
+    const int nx = (int)g.n[0], ny = (int)g.n[1], nz = (int)g.n[2];
+    auto blocks = [&](int ax) { return (unsigned int)((n / g.n[ax] + 63) / 64); };
+    Deriche c;
+    if (!rc) rc = deriche_zero_order(sigma_mm[2], g.sp[2], c);
     if (!rc) {
-        k_f64_to_f32<<<blocks, 256, 0, ctx->stream>>>(vol, out->d, n);
-        rc = check_launch(ctx, "k_f64_to_f32");
+        k_deriche<float, double><<<blocks(2), 64, 0, ctx->stream>>>(img->d, tmp, z, nx, ny, nz, 2, c);
+        rc = check_launch(ctx, "k_deriche");
     }
-    dev_free(ctx, vol, sizeof(double) * n);
+    if (!rc) rc = deriche_zero_order(sigma_mm[0], g.sp[0], c);
+    if (!rc) {
+        k_deriche<double, double><<<blocks(0), 64, 0, ctx->stream>>>(z, tmp, x, nx, ny, nz, 0, c);
+        rc = check_launch(ctx, "k_deriche");
+    }
+    if (!rc) rc = deriche_zero_order(sigma_mm[1], g.sp[1], c);
+    if (!rc) {
+        k_deriche<double, float><<<blocks(1), 64, 0, ctx->stream>>>(x, tmp, out->d, nx, ny, nz, 1, c);
+        rc = check_launch(ctx, "k_deriche");
+    }
     dev_free(ctx, tmp, sizeof(double) * n);
-    dev_free(ctx, nxt, sizeof(double) * n);
+    if (z) dev_free(ctx, z, sizeof(double) * n);
+    if (x) dev_free(ctx, x, sizeof(double) * n);
     return rc;
 }
 

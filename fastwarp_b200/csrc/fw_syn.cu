@@ -18,6 +18,7 @@
 // The host launches one graph and reads the records back once per level.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <chrono>
 #include <cstdio>
@@ -247,6 +248,14 @@ int enqueue_invert_pair(fw_ctx* ctx, bool graph, fw_field* const field[2], fw_fi
 
 unsigned int blocks256(long long n) { return (unsigned int)((n + 255) / 256); }
 
+// How many sides one launch of the smoothing and the composition takes: they hand a field on through
+// L2 (126 MB), and two fields that do not fit go one side after the other (193 x 229 x 193, 102 MB a
+// field: 1738 us an iteration with both in one launch, 1718 in turn; 96 x 114 x 96, 13 MB: 357 and
+// 361).
+int sides_together(const HostGrid& g) {
+    return 2 * 12 * plane_stride(g.count()) > (100LL << 20) ? 1 : 2;
+}
+
 // The kernels of one iteration (syn.rs:890-958) on ctx->stream.
 int enqueue_iteration(fw_ctx* ctx, bool graph, const fw_syn_recipe* r, Level& L,
                       const std::vector<const fw_image*>& fs,
@@ -332,18 +341,24 @@ int enqueue_iteration(fw_ctx* ctx, bool graph, const fw_syn_recipe* r, Level& L,
     fw_field* work[2] = {L.sF, L.sM};
     fw_field* field[2] = {L.F, L.M};
     fw_field* inverse[2] = {L.Fi, L.Mi};
-    if (r->update_field_variance > 0.0) {
-        bool in_tmp = false;
-        FW_TRY(launch_smooth_pair(ctx, u, work, r->update_field_variance, d.max_bits, &in_tmp));
-        if (in_tmp)
-            for (int s = 0; s < 2; ++s) std::swap(u[s], work[s]);
-    } else {
-        for (int s = 0; s < 2; ++s) FW_TRY(launch_max_norm(ctx, u[s], d.max_bits + s));
+    // The composition is in place: every voxel reads its own field value and the update elsewhere.
+    const int sides = sides_together(L.grid);
+    for (int s = 0; s < 2; s += sides) {
+        if (r->update_field_variance > 0.0) {
+            bool in_tmp = false;
+            FW_TRY(launch_smooth_sides(ctx, u + s, work + s, sides, r->update_field_variance,
+                                       d.max_bits + s, &in_tmp));
+            for (int q = s; q < s + sides && in_tmp; ++q) std::swap(u[q], work[q]);
+        } else {
+            for (int q = s; q < s + sides; ++q) FW_TRY(launch_max_norm(ctx, u[q], d.max_bits + q));
+        }
+        if (sides == 2)
+            FW_TRY(launch_compose_pair(ctx, u, field, d.max_bits, r->gradient_step));
+        else
+            FW_TRY(launch_compose(ctx, u[s], field[s], field[s], d.max_bits + s, r->gradient_step));
     }
     L.uF = u[0];
     L.uM = u[1];
-    // compose in place: every voxel reads its own field value and the update elsewhere
-    FW_TRY(launch_compose_pair(ctx, u, field, d.max_bits, r->gradient_step));
     if (r->total_field_variance > 0.0) {
         for (int s = 0; s < 2; ++s) {
             FW_TRY(launch_smooth(ctx, field[s], L.T, r->total_field_variance, nullptr, work[s]));
@@ -624,9 +639,10 @@ int check_status(int status, bool masked) {
 }
 
 // Kernels per iteration outside the inversion bodies (for the launch counter).
-int kernels_per_iteration(const fw_syn_recipe* r, int mask_warps, bool prior) {
+int kernels_per_iteration(const fw_syn_recipe* r, int mask_warps, bool prior, int sides) {
     int k = r->channels * (prior ? 3 : 2) + (r->channels > 1 ? 2 * r->channels + 2 : 0) +
-            2 /*two-pass smoothing or max*/ + 1 /*compose*/ +
+            (r->update_field_variance > 0.0 && sides == 1 ? 4 : 2) /*two-pass smoothing, or max*/ +
+            (sides == 1 ? 2 : 1) /*compose*/ +
             (r->total_field_variance > 0.0 ? 4 : 0) + 1 /*inversion inits*/ + 1 /*record*/ +
             mask_warps + (mask_warps == 2 ? 1 : 0) /*product*/;
     for (int c = 0; c < r->channels; ++c)
@@ -772,10 +788,9 @@ int syn_run_device(fw_ctx* ctx, const fw_syn_recipe* r, const fw_image* const* f
                 FW_CUDA(cudaMemsetAsync(nx[q]->d, 0, nx[q]->bytes, ctx->stream));
             } else if (prev.same(lg)) {
                 FW_CUDA(cudaMemcpyAsync(nx[q]->d, st[q]->d, nx[q]->bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-            } else {
-                rc = launch_resample(ctx, st[q], nx[q]);
             }
         }
+        if (!rc && have_prev && !prev.same(lg)) rc = launch_resample(ctx, st, nx, 4);
         if (rc) {
             for (auto* f : nx) fw_field_free(f);
             break;
@@ -829,15 +844,18 @@ int syn_run_device(fw_ctx* ctx, const fw_syn_recipe* r, const fw_image* const* f
                 FW_CUDA(cudaMemcpy(all.data(), rs.d.trace, sizeof(fw_syn_iteration) * done,
                                    cudaMemcpyDeviceToHost));
             // the kernels the level graphs ran (direct launches are counted as they are made):
-            // every iteration's kernels, three per inversion body of the two sides, one level init
-            // per level
+            // every iteration's kernels, three per inversion body of the two sides (the plain bodies
+            // are launched whether they run or not), one level init per level
             for (int q = 0; q < done && graphs; ++q) {
+                HostGrid g;
+                FW_TRY(level_grid(r, fg, all[q].level, g));
                 for (int s = 0; s < 2; ++s)
                     ctx->stats.kernel_launches +=
-                        3 * (uint64_t)std::max(all[q].inversions[s].iterations,
-                                               all[q].inversions[s + 2].iterations);
-                ctx->stats.kernel_launches += kernels_per_iteration(
-                    r, (fixed_mask ? 1 : 0) + (moving_mask ? 1 : 0), prior != nullptr);
+                        3 * (uint64_t)std::max({plain_bodies(g), all[q].inversions[s].iterations,
+                                                all[q].inversions[s + 2].iterations});
+                ctx->stats.kernel_launches +=
+                    kernels_per_iteration(r, (fixed_mask ? 1 : 0) + (moving_mask ? 1 : 0),
+                                          prior != nullptr, sides_together(g));
             }
             if (graphs) ctx->stats.kernel_launches += (uint64_t)graph_levels;
             if (records && cap > 0)
