@@ -424,8 +424,8 @@ int fw_mi_level_num_valid(const fw_mi_level* level, int64_t* out);
 /* Profiling (crates/fastwarp-gpu/src/profiler.rs:8-60, per-op device timestamps): after one
  * evaluation at `t`, times `reps` back-to-back launches of each pass of the level with CUDA events
  * on the context's stream and writes the mean milliseconds per launch and the algorithmic bytes
- * per launch of [0] the joint histogram (clear + k_mi_hist), [1] ComputeResults (k_mi_finish),
- * [2] the gradient moments (k_mi_deriv). A pass's bytes are the 16-byte sample records and the
+ * per launch of [0] the joint histogram (clear + k_mi_hist), [1] ComputeResults (k_mi_finish; an
+ * evaluation has it done by the histogram pass's last block), [2] the gradient moments (k_mi_deriv). A pass's bytes are the 16-byte sample records and the
  * moving image's gathers, min(4 Nm, 32 S) for S samples on Nm moving voxels. */
 int fw_mi_level_time(fw_mi_level* level, const fw_linear_transform* t, int32_t reps,
                      double ms[3], double bytes[3]);

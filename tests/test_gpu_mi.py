@@ -164,6 +164,39 @@ def test_dense_histogram_merges_its_words_before_they_overflow(backend):
     assert np.allclose(out[0], out[1], rtol=1e-12, atol=0.0)
 
 
+@pytest.mark.parametrize("where", ["jittered", "centres", "faces"])
+def test_gradient_on_an_axis_aligned_image_matches(backend, where):
+    """The gradient from a sample's own corners and four more an axis: inside the image, at voxel
+    centres (weights of zero) and in the outermost voxels (corners outside), the last two by the
+    general probes."""
+    size, spacing, origin = (19, 17, 15), (1.0, 2.0, 0.8), (1.0, -2.0, 3.0)
+    og, g, f, m, kept, fbin, b = setup(size, spacing, origin, np.eye(3), seed=8)
+    rng = np.random.default_rng(12)
+    n = np.array(size)
+    if where != "jittered":
+        if where == "centres":
+            idx = np.stack([rng.integers(2, k - 2, 600) for k in n], 1).astype(float)
+        else:
+            idx = rng.uniform(0.3, n - 1.3, (600, 3))
+            side = rng.integers(0, 3, 600)
+            far = rng.random(600) < 0.5
+            depth = rng.uniform(0.02, 0.9, 600)
+            idx[np.arange(600), side] = np.where(far, n[side] - 1 - depth, depth)
+        pts = np.asarray(origin) + idx * np.asarray(spacing)
+        kept, fbin, b = O.prepare_samples(og, f, og, m, pts, 32)
+    level = CudaLinearEngine(backend).prepare_level(g, m, kept, fbin, b)
+    kw = dict(kind="affine", parameters=[1, 0, 0, 0, 1, 0, 0, 0, 1, 0, 0, 0], center=(0, 0, 0))
+    if where != "centres":
+        kw["parameters"] = [1.01, 0.02, 0, -0.01, 0.99, 0, 0.01, 0, 1.0, 0.1, -0.2, 0.05]
+        kw["center"] = tuple(kept.mean(0))
+    v, d = level.value_and_derivative(linear_transform(**kw))
+    wv, wd, wn, _ = O.mi_evaluate(b, og, m, kept, fbin, O.linear_transform(**kw))
+    assert level.num_valid() == wn
+    # float32 sample offsets and interpolation: about 1e-6 of the difference of two values
+    assert abs(v - wv) <= 1e-5 * abs(wv)
+    assert np.linalg.norm(d - wd) <= 5e-4 * np.linalg.norm(wd)
+
+
 def test_all_samples_outside_is_an_error(backend):
     from fastwarp_b200 import FastwarpError
     og, g, f, m, kept, fbin, b = setup()
