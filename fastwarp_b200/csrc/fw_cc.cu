@@ -54,7 +54,8 @@ struct CcArgs {
     float ispf[3];      // the same in float32
     int mode;           // the kernel's MODE
     // the probe at -half (p = 2d) and +half (2d + 1) a spacing along physical axis d, relative to
-    // its voxel: index offset of its lower corner (-1 or 0) and weights of the upper one
+    // its voxel: index offset of its lower corner (-1 or 0; 1 only where the weight is 0, a probe on
+    // the neighbour itself: axes permuted and one spacing twice another) and weights of the upper one
     signed char base[6][3];
     float weight[6][3];
 };
@@ -524,7 +525,7 @@ __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
                 const float wx = a.weight[p][0], wy = a.weight[p][1], wz = a.weight[p][2];
                 const int at = a.base[p][0] + L::RX * a.base[p][1];
                 const int ox = wx > 0.0f ? 1 : 0, oy = wy > 0.0f ? L::RX : 0;
-                const bool low = a.base[p][2] < 0;
+                const int slice = a.base[p][2];
                 auto plane = [&](const float2* s) {
                     const float2 v00 = s[at], v10 = s[at + ox], v01 = s[at + oy], v11 = s[at + oy + ox];
                     const float fx0 = fmaf(v10.x - v00.x, wx, v00.x);
@@ -533,10 +534,10 @@ __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
                     const float mx1 = fmaf(v11.y - v01.y, wx, v01.y);
                     return make_float2(fmaf(fx1 - fx0, wy, fx0), fmaf(mx1 - mx0, wy, mx0));
                 };
-                const float2 a0 = plane(low ? below : cs);
+                const float2 a0 = plane(slice < 0 ? below : (slice == 0 ? cs : above));
                 v[p & 1] = a0;
                 if (wz > 0.0f) {
-                    const float2 a1 = plane(low ? cs : above);
+                    const float2 a1 = plane(slice < 0 ? cs : above);
                     v[p & 1] = make_float2(fmaf(a1.x - a0.x, wz, a0.x), fmaf(a1.y - a0.y, wz, a0.y));
                 }
                 if (p & 1) {

@@ -111,6 +111,32 @@ def test_the_default_tile_shapes_without_the_autotuner(backend):
     compare(backend, r, fixed, subjects, batch)
 
 
+def test_a_batch_on_a_permuted_template_matches_the_oracle(backend):
+    """A template whose axes are permuted, one spacing twice another: the CC pair's probes of a
+    batch lie on neighbouring voxels themselves. One iteration against the oracle's (with a step off
+    0.1 voxel, the inversion's tolerance on its largest error: there one rounding decides a body more)."""
+    import oracle as O
+    from cases import image
+    from fastwarp_b200 import make_grid
+    case = dict(size=(35, 21, 19), seed=23)
+    geo = ((2.0, 1.0, 1.0), (3.0, -4.0, 5.0), np.array([[0, 0, 1.0], [1, 0, 0], [0, 1, 0]]))
+    g, og = make_grid(case["size"], *geo), O.make_grid(case["size"], *geo)
+    f = image(case)
+    ms = [image(case, seed_offset=k) for k in (1, 2)]
+    r = recipe(gradient_step=0.25, iterations=[1], shrink_factors=[1], smoothing_sigmas=[0.0],
+               channel_weights=[1.0])
+    up = [backend.upload_image(g, a.astype(np.float32)) for a in (f, *ms)]
+    batch = run_syn_batch(backend, r, up[:1], [([m], None) for m in up[1:]])
+    assert batch.statuses == [0, 0]
+    for m, got in zip(ms, batch.subjects):
+        w, iw, recs, _ = O.syn_run(O.syn_recipe(0.25, 3.0, 0.0, 2, (1,), (1,), (0.0,), False, -1.0),
+                                   og, [f], og, [m])
+        assert abs(got.iterations[0]["energy"] - recs[0].energy) <= 1e-5 * abs(recs[0].energy)
+        # the ops' bounds: 1e-4 of the largest displacement for the derivative and the inversion
+        assert np.abs(got.warp - w).max() <= 3e-4 * np.abs(w).max()
+        assert np.abs(got.inverse_warp - iw).max() <= 3e-4 * np.abs(iw).max()
+
+
 def test_batch_recipe_limits_are_refused(backend):
     from fastwarp_b200 import FastwarpError
     g, fixed, subjects = batch_subjects(backend, 1, template_shape=(24, 24, 24), dims=(20, 24),

@@ -210,6 +210,39 @@ def test_cc_every_kind_of_grid_matches(backend, spacing, oblique, radius):
             assert worst(backend.download_field(d), e) <= 1e-4 * np.abs(e).max()
 
 
+SAGITTAL = [[0, 0, 1], [1, 0, 0], [0, 1, 0]]
+
+
+@pytest.mark.parametrize("spacing", [(1.0, 1.0, 1.0), (1.0, 1.0, 0.5), (2.0, 1.0, 1.0), (0.9, 0.9, 0.45),
+                                     (0.8, 0.8, 0.4), (1.2, 1.0, 1.1)])
+@pytest.mark.parametrize("direction", [SAGITTAL, [[0, -1, 0], [0, 0, -1], [1, 0, 0]],
+                                       [[1, 0, 0], [0, 0, 1], [0, -1, 0]], [[0, 1, 0], [1, 0, 0], [0, 0, 1]],
+                                       np.diag([-1, -1, 1]), np.diag([1, 1, -1])])
+def test_cc_on_permuted_and_flipped_axes_matches(backend, direction, spacing):
+    """The orientations of scanners: probes along an index axis that is not their physical one. With one
+    spacing twice another a probe lies on a neighbouring voxel itself, one up or one down."""
+    case = dict(CASES["awkward_oblique"], size=(35, 13, 11), spacing=spacing, direction=direction)
+    og, g = grid_of(case), fgrid(case)
+    fimg, mimg = image(case), image(case, seed_offset=3)
+    fi = backend.upload_image(g, fimg.astype(np.float32))
+    mi = backend.upload_image(g, mimg.astype(np.float32))
+    valid = ball_mask(case)
+    vi = backend.upload_image(g, valid.astype(np.float32))
+    want = O.cc_pair(og, fimg, mimg, 2)
+    got = [(backend.cc_value_derivative_pair(fi, mi, 2), want),
+           (backend.cc_value_derivative_pair_masked(fi, mi, vi, 2),
+            O.cc_pair(og, fimg, mimg, 2, valid=valid))]
+    N.check(N.lib().fw_set_cc_window_sums(1))  # the compensated float32 sums
+    try:
+        got.append((backend.cc_value_derivative_pair(fi, mi, 2), want))
+    finally:
+        N.check(N.lib().fw_set_cc_window_sums(0))
+    for pair, expected in got:
+        for (v, d), (w, e) in zip(pair, expected):
+            assert rel(v, w) <= 1e-5
+            assert worst(backend.download_field(d), e) <= 1e-4 * np.abs(e).max()
+
+
 def ball_mask(case):
     """metric/cc.rs:465-473's mask shape on the case grid: out of a ball, the first x plane and a
     corner strip; the inside value is 3 (any non-zero value counts)."""

@@ -19,11 +19,16 @@ from fastwarp_b200 import _native as N
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("name", ["awkward_aligned", "awkward_oblique"])
+# axes permuted with one spacing twice another: probes on the neighbouring voxels themselves
+PERMUTED = dict(CASES["awkward_oblique"], size=(35, 13, 11), spacing=(2.0, 1.0, 1.0),
+                direction=np.array([[0, 0, 1.0], [1, 0, 0], [0, 1, 0]]), radius=2)
+
+
+@pytest.mark.parametrize("name", ["awkward_aligned", "awkward_oblique", "permuted"])
 def test_the_allocation_free_cc_pair_matches_the_ordinary_entry_point(name):
     import torch
 
-    case = CASES[name]
+    case = dict(CASES, permuted=PERMUTED)[name]
     g = make_grid(case["size"], case["spacing"], case["origin"], case["direction"])
     og = O.make_grid(case["size"], case["spacing"], case["origin"], case["direction"])
     r = case["radius"]
@@ -56,8 +61,10 @@ def test_the_allocation_free_cc_pair_matches_the_ordinary_entry_point(name):
             assert abs(np.sqrt(n1) - np.sqrt((want1 ** 2).sum())) <= 1e-5 * np.sqrt((want1 ** 2).sum())
             assert abs(np.sqrt(n2) - np.sqrt((want2 ** 2).sum())) <= 1e-5 * np.sqrt((want2 ** 2).sum())
         # and both agree with the f64 oracle
-        (w1, _), _ = O.cc_pair(og, fimg, mimg, r)
+        (w1, e1), (_, e2) = O.cc_pair(og, fimg, mimg, r)
         assert abs(value - w1) <= 1e-5 * abs(w1)
+        assert np.abs(got1 - e1).max() <= 1e-4 * np.abs(e1).max()
+        assert np.abs(got2 - e2).max() <= 1e-4 * np.abs(e2).max()
 
 
 def test_the_allocation_free_cc_pair_rejects_grids_beyond_its_scratch():
