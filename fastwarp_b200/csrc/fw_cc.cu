@@ -19,14 +19,18 @@
 // The pair's whole call at 193 x 229 x 193, r = 4: 400 us with 64 additions an x group and 20 a y
 // group, window counters, and the face tests and float64 scaling of the gradients at every voxel;
 // 325 us now. Masked, r = 3, 181 x 217 x 165 on a rotated grid with every probe from global memory in
-// float64: 458 us; 328 us with the probes' common corners and weights on the raw slices.
+// float64: 458 us; 289 us with the probes' common corners and weights on the raw slices, the faces
+// included (328 with every probe of a face's warp from global memory; unmasked 64 x 217 x 165, where
+// every warp holds a face, 311 us with all probes from global memory, 386 with them at the faces, 139).
 // Measured and dropped: z sums in registers (spills at three CTAs: 521 us), 16 rows a tile with one
 // or two voxels a thread (363-424 us), two CTAs an SM without spills (374 us), thinner z chunks on
 // coarse grids (no change: the call's fixed cost).
 #include <cuda_runtime.h>
 
-#include <cfloat>
+#include <algorithm>
 #include <atomic>
+#include <cfloat>
+#include <cmath>
 #include <cstring>
 
 #include "fw_internal.cuh"
@@ -41,7 +45,7 @@ constexpr int CC_NT = 256;       // threads of a CTA
 
 // Kinds of grids by their central differences: CC_AXES an identity direction with every 1 / spacing
 // a float32 (1, 2, 0.5, 0.8 mm ...); CC_ROTATED another direction whose probes stay within one voxel
-// of theirs; CC_ANY any of these and the rest (0.9 mm, a rotated grid of very unequal spacings).
+// of theirs; CC_ANY the rest (an identity direction at 0.9 mm, a rotated grid of very unequal spacings).
 enum CcMode { CC_ANY, CC_AXES, CC_ROTATED };
 
 struct CcArgs {
@@ -49,7 +53,6 @@ struct CcArgs {
     long long ps;       // plane stride of the derivative fields
     int zchunk;         // slices per CTA
     int identity_dir;   // direction is the identity: axis-aligned probes
-    int stencil;        // rotated grid whose probes stay within one voxel: `probe` holds them
     double isp[3];      // 1 / spacing (the central difference's denominator)
     float ispf[3];      // the same in float32
     int mode;           // the kernel's MODE
@@ -58,6 +61,10 @@ struct CcArgs {
     // the neighbour itself: axes permuted and one spacing twice another) and weights of the upper one
     signed char base[6][3];
     float weight[6][3];
+    // at a face of index axis r: the physical axes (bit d) whose probes reach more than half a voxel
+    // along r and so leave the buffer there, and the one (or 3, none) whose probes end on the half
+    // voxel, where the reference's rounding decides
+    unsigned char out[3], edge[3];
 };
 
 // Shared-memory layout (dynamic): the z-window sums of every halo column, [5][HY][HX] double
@@ -184,11 +191,21 @@ __device__ __forceinline__ void window_sums(Load load, Store store) {
     }
 }
 
-// The exact probes of a rotated grid's faces, called rather than inlined: their float64 registers
-// would be spilled for in the tile's loop.
+// The exact probes, called rather than inlined: their float64 registers would be spilled for in the
+// tile's loop.
 __device__ __noinline__ void cc_exact_gradient(const float* __restrict__ img, const DevGrid& g,
                                                int x, int y, int z, float out[3]) {
     central_difference_exact(img, g, x, y, z, out);
+}
+
+// Whether a probe of voxel (x, y, z) along physical axis d is outside the buffer along index axis r,
+// by the reference's own arithmetic.
+__device__ __noinline__ bool cc_probe_outside(const DevGrid& g, int x, int y, int z, int d, int r,
+                                              int n) {
+    double a[3], b[3];
+    probe_index(g, x, y, z, d, -1.0, a);
+    probe_index(g, x, y, z, d, +1.0, b);
+    return !(a[r] >= -0.5 && a[r] < (double)n - 0.5 && b[r] >= -0.5 && b[r] < (double)n - 0.5);
 }
 
 // One tile (bx, by, bz) of the CC pair: writes the tile's derivative voxels and leaves the
@@ -357,6 +374,20 @@ __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
         if (!inside(x, y0, nz - 1, 2, nz)) ok &= ~4u;
         if (!inside(x, y, z0, 1, ny)) ok &= ~8u;
     }
+    // rotated grids: the physical axes (bits 0-2) whose difference is zero at the voxel's x and y
+    // faces, then (bits 4-6, 8-10) at the first and the last slice; a probe that ends on the half
+    // voxel depends on the coordinate along that axis alone (cc_args)
+    unsigned int gone = 0;
+    if (MODE == CC_ROTATED && own) {
+        auto face = [&](int r, int n, int i, int j, int k) {
+            unsigned int m = a.out[r];
+            if (a.edge[r] < 3 && cc_probe_outside(a.g, i, j, k, a.edge[r], r, n)) m |= 1u << a.edge[r];
+            return m;
+        };
+        if (x == 0 || x == nx - 1) gone |= face(0, nx, x, y0, z0);
+        if (y == 0 || y == ny - 1) gone |= face(1, ny, x0, y, z0);
+        gone |= face(2, nz, x0, y0, 0) << 4 | face(2, nz, x0, y0, nz - 1) << 8;
+    }
     // analytic voxel count of the clamped window along x and y
     const int cxy = own ? (min(x + R, nx - 1) - max(x - R, 0) + 1) *
                               (min(y + R, ny - 1) - max(y - R, 0) + 1) : 1;
@@ -515,8 +546,10 @@ __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
             diff(0, ok & 1u, cs[-1], cs[1]);
             diff(1, ok & 8u, cs[-L::RX], cs[L::RX]);
             diff(2, (z > 0 || (ok & 2u)) && (z < nz - 1 || (ok & 4u)), lo, hi);
-        } else if ((MODE == CC_ROTATED || a.stencil) && x > 0 && x < nx - 1 && y > 0 && y < ny - 1 && z > 0 && z < nz - 1) {
-            // a rotated grid: off the faces every probe's corners and weights are the same
+        } else if (MODE == CC_ROTATED) {
+            // a rotated grid: every probe's corners and weights are the same, and a corner outside the
+            // buffer is the clamped ring's face voxel, which lin_axis reads there
+            const unsigned int no = gone | (z == 0 ? gone >> 4 : 0u) | (z == nz - 1 ? gone >> 8 : 0u);
             const float2* below = raw + ((z - 1) & 3) * L::RXY + oslot;
             const float2* above = raw + ((z + 1) & 3) * L::RXY + oslot;
             float2 v[2];
@@ -543,6 +576,7 @@ __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
                 if (p & 1) {
                     gf[p >> 1] = (float)((double)(v[1].x - v[0].x) * a.isp[p >> 1]);
                     gm[p >> 1] = (float)((double)(v[1].y - v[0].y) * a.isp[p >> 1]);
+                    if (no >> (p >> 1) & 1u) gf[p >> 1] = gm[p >> 1] = 0.0f;
                 }
             }
         } else {
@@ -733,8 +767,13 @@ int launch_radius(fw_ctx* ctx, const CcArgs& a, int radius, const float* f, cons
 #define FW_CC_RADIUS(RR)                                                                         \
     case RR:                                                                                    \
         if constexpr (!MK)                                                                      \
-            if (c32) return launch_r<RR, CC_TY, false, CC_ANY, SumC32>(ctx, a, f, m, v, df, dm,  \
-                                                                     d_result, want_norms);     \
+            if (c32)                                                                            \
+                return a.mode == CC_ROTATED                                                     \
+                           ? launch_r<RR, CC_TY, false, CC_ROTATED, SumC32>(                    \
+                                 ctx, a, f, m, v, df, dm, d_result, want_norms)                 \
+                           : launch_r<RR, CC_TY, false, CC_ANY, SumC32>(ctx, a, f, m, v, df,    \
+                                                                        dm, d_result,           \
+                                                                        want_norms);            \
         if (a.mode == CC_AXES)                                                                  \
             return launch_r<RR, CC_TY, MK, CC_AXES>(ctx, a, f, m, v, df, dm, d_result,          \
                                                     want_norms);                                \
@@ -801,7 +840,35 @@ CcArgs cc_args(const HostGrid& g, long long ps) {
             if (g.dir[r * 3 + c] != (r == c ? 1.0 : 0.0)) a.identity_dir = 0;
     const bool exact = (double)a.ispf[0] == a.isp[0] && (double)a.ispf[1] == a.isp[1] &&
                        (double)a.ispf[2] == a.isp[2];
-    a.stencil = !a.identity_dir;
+    bool stencil = !a.identity_dir;
+    // How far rounding can move a probe's index: a few float64 units of the largest coordinate in
+    // voxels (and no less than 1e-9).
+    double reach = 0.0, least = g.sp[0];
+    for (int d = 0; d < 3; ++d) {
+        reach = std::max(reach, std::fabs(g.org[d]));
+        least = std::min(least, g.sp[d]);
+    }
+    for (int d = 0; d < 3; ++d) reach += (double)g.n[d] * g.sp[d];
+    const double slack = std::max(1e-9, 256.0 * DBL_EPSILON * reach / least);
+    for (int r = 0; r < 3; ++r) {
+        a.edge[r] = 3;
+        for (int d = 0; d < 3; ++d) {
+            const double h = 0.5 * g.sp[d] * std::fabs(g.inv[r * 3 + d]);
+            if (h > 0.5 + slack) {
+                a.out[r] |= (unsigned char)(1u << d);
+            } else if (h >= 0.5 - slack) {
+                // on the half voxel: decided once a column, if index r follows physical axis d alone
+                // and d index r alone (the other terms of the probe's index are exact zeros)
+                bool alone = a.edge[r] == 3;
+                for (int q = 0; q < 3; ++q) {
+                    if (q != d && g.inv[r * 3 + q] != 0.0) alone = false;
+                    if (q != r && g.dir[d * 3 + q] != 0.0) alone = false;
+                }
+                if (alone) a.edge[r] = (unsigned char)d;
+                else stencil = false;
+            }
+        }
+    }
     for (int p = 0; p < 6; ++p)
         for (int r = 0; r < 3; ++r) {
             // index offset along axis r of the probe along physical axis p / 2
@@ -814,13 +881,13 @@ CcArgs cc_args(const HostGrid& g, long long ps) {
             } else if (w < 1e-12) {
                 w = 0.0;
             }
-            if (!(base >= -1.0 && base + (w > 0.0 ? 1.0 : 0.0) <= 1.0)) a.stencil = 0;
+            if (!(base >= -1.0 && base + (w > 0.0 ? 1.0 : 0.0) <= 1.0)) stencil = false;
             else {
                 a.base[p][r] = (signed char)base;
                 a.weight[p][r] = (float)w;
             }
         }
-    a.mode = a.identity_dir ? (exact ? CC_AXES : CC_ANY) : (a.stencil ? CC_ROTATED : CC_ANY);
+    a.mode = a.identity_dir ? (exact ? CC_AXES : CC_ANY) : (stencil ? CC_ROTATED : CC_ANY);
     return a;
 }
 
@@ -856,15 +923,11 @@ int launch_cc_pair_batch(fw_ctx* ctx, const HostGrid& g, long long ps, int radiu
     a.zchunk = zchunk;
 #define FW_CC_BATCH(RR)                                                                          \
     case RR:                                                                                    \
-        return a.mode == CC_AXES                                                                \
-                   ? launch_cc_batch_r<RR, CC_AXES>(ctx, a, L, blocks, fimg, mimg, img_stride,  \
-                                                    d_fixed, d_moving, field_stride, partials,  \
-                                                    part_stride, counter, result,               \
-                                                    result_stride, want_norms)                  \
-                   : launch_cc_batch_r<RR, CC_ANY>(ctx, a, L, blocks, fimg, mimg, img_stride,   \
-                                                   d_fixed, d_moving, field_stride, partials,   \
-                                                   part_stride, counter, result, result_stride, \
-                                                   want_norms);
+        return (a.mode == CC_AXES      ? launch_cc_batch_r<RR, CC_AXES>                         \
+                : a.mode == CC_ROTATED ? launch_cc_batch_r<RR, CC_ROTATED>                      \
+                                       : launch_cc_batch_r<RR, CC_ANY>)(                        \
+            ctx, a, L, blocks, fimg, mimg, img_stride, d_fixed, d_moving, field_stride,         \
+            partials, part_stride, counter, result, result_stride, want_norms);
     switch (radius) {
         FW_CC_BATCH(1)
         FW_CC_BATCH(2)
@@ -1080,11 +1143,10 @@ extern "C" int fw_cc_value_derivative_pair_noalloc(const fw_grid* grid, const fl
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define FW_CC_NOALLOC(RR)                                                                        \
     case RR:                                                                                    \
-        return a.mode == CC_AXES                                                                \
-                   ? noalloc_launch<RR, CC_TY, CC_AXES>(a, num_sms, fixed, moving, d_fixed,     \
-                                                        d_moving, result, s, st)                \
-                   : noalloc_launch<RR, CC_TY, CC_ANY>(a, num_sms, fixed, moving, d_fixed,      \
-                                                       d_moving, result, s, st);
+        return (a.mode == CC_AXES      ? noalloc_launch<RR, CC_TY, CC_AXES>                     \
+                : a.mode == CC_ROTATED ? noalloc_launch<RR, CC_TY, CC_ROTATED>                  \
+                                       : noalloc_launch<RR, CC_TY, CC_ANY>)(                    \
+            a, num_sms, fixed, moving, d_fixed, d_moving, result, s, st);
     switch (radius) {
         FW_CC_NOALLOC(1)
         FW_CC_NOALLOC(2)

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import oracle as O
-from cases import (CASES, continuous_index, edge_distance, field, grid_of, image,
+from cases import (CASES, continuous_index, edge_distance, field, grid_of, image, rot_x, rot_z,
                    vector_at, voxel_points)
 from fastwarp_b200 import _native as N
 from fastwarp_b200.backend import make_affine, make_grid
@@ -241,6 +241,39 @@ def test_cc_on_permuted_and_flipped_axes_matches(backend, direction, spacing):
         for (v, d), (w, e) in zip(pair, expected):
             assert rel(v, w) <= 1e-5
             assert worst(backend.download_field(d), e) <= 1e-4 * np.abs(e).max()
+
+
+def rot_y(a):
+    c, s = np.cos(a), np.sin(a)
+    return np.array([[c, 0.0, s], [0.0, 1.0, 0.0], [-s, 0.0, c]])
+
+
+@pytest.mark.parametrize("kind", ["one_axis", "third_turn", "permuted", "oblique"])
+def test_cc_probes_at_the_faces_of_rotated_grids_match(backend, kind):
+    """Grids of two voxels an axis up to a few, where most voxels are at a face: probes that leave the
+    buffer, that stay inside and that end on its edge, turned about one axis (probes of the others end
+    on the edge), by a sixth of a turn (with one spacing twice another these do too, in no one
+    coordinate), permuted and oblique."""
+    rng = np.random.default_rng(7)
+    for k in range(16):
+        a = rng.uniform(-3.0, 3.0)
+        turn = (rot_x, rot_y, rot_z)[k % 3]
+        direction = {"one_axis": turn(a), "third_turn": turn(np.pi / 3 * rng.integers(1, 6)),
+                     "permuted": np.eye(3)[rng.permutation(3)] * rng.choice([-1.0, 1.0], 3),
+                     "oblique": rot_z(a) @ rot_x(0.3 * a)}[kind]
+        size = [int(v) for v in rng.integers(2, 9, 3)]
+        size[k % 3] = int(rng.choice([2, 9, 33, 40]))
+        case = dict(CASES["awkward_oblique"], size=tuple(size), direction=direction,
+                    origin=tuple(rng.uniform(-300.0, 300.0, 3)),
+                    spacing=tuple(rng.choice([0.5, 0.8, 0.9, 1.0, 1.0, 2.0], 3)))
+        og, g = grid_of(case), fgrid(case)
+        fimg, mimg = image(case, noise=0.2), image(case, seed_offset=3, noise=0.2)
+        fi = backend.upload_image(g, fimg.astype(np.float32))
+        mi = backend.upload_image(g, mimg.astype(np.float32))
+        for (v, d), (w, e) in zip(backend.cc_value_derivative_pair(fi, mi, 2),
+                                  O.cc_pair(og, fimg, mimg, 2)):
+            assert rel(v, w) <= 1e-5, (k, case)
+            assert worst(backend.download_field(d), e) <= 1e-4 * np.abs(e).max(), (k, case)
 
 
 def ball_mask(case):
