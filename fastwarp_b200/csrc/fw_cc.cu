@@ -43,16 +43,18 @@ constexpr int TX = 32;
 constexpr int CC_TY = 8;         // rows of a tile
 constexpr int CC_NT = 256;       // threads of a CTA
 
-// Kinds of grids by their central differences: CC_AXES an identity direction with every 1 / spacing
-// a float32 (1, 2, 0.5, 0.8 mm ...); CC_ROTATED another direction whose probes stay within one voxel
-// of theirs; CC_ANY the rest (an identity direction at 0.9 mm, a rotated grid of very unequal spacings).
-enum CcMode { CC_ANY, CC_AXES, CC_ROTATED };
+// Kinds of grids by their central differences, a kernel each: CC_AXES an identity direction with every
+// 1 / spacing a float32 (1, 2, 0.5, 0.8 mm ...); CC_AXES64 one with others (0.9, 0.7 mm), whose
+// differences are scaled in float64; CC_ROTATED another direction whose probes stay within one voxel
+// of theirs; CC_EXACT the rest (very unequal spacings), every probe by itself. One kernel of the
+// second and the last spilled the call's registers in the loop: 0.9 mm at 193 x 229 x 193 393 us (r 3), masked
+// 500 (r 4); apart 326 and 388.
+enum CcMode { CC_EXACT, CC_AXES, CC_AXES64, CC_ROTATED };
 
 struct CcArgs {
     DevGrid g;
     long long ps;       // plane stride of the derivative fields
     int zchunk;         // slices per CTA
-    int identity_dir;   // direction is the identity: axis-aligned probes
     double isp[3];      // 1 / spacing (the central difference's denominator)
     float ispf[3];      // the same in float32
     int mode;           // the kernel's MODE
@@ -191,11 +193,38 @@ __device__ __forceinline__ void window_sums(Load load, Store store) {
     }
 }
 
-// The exact probes, called rather than inlined: their float64 registers would be spilled for in the
-// tile's loop.
-__device__ __noinline__ void cc_exact_gradient(const float* __restrict__ img, const DevGrid& g,
-                                               int x, int y, int z, float out[3]) {
-    central_difference_exact(img, g, x, y, z, out);
+// The exact central differences of both images (interp.rs:96-120 at voxel (x, y, z)), the probes'
+// float64 indices formed once for the two. Inlined into the loop of the one kind of grid that needs it:
+// as a call, its operands and the loop's go through local memory (193 x 229 x 193, spacings 0.5 / 8 /
+// 0.7 mm turned, r 4: 1749 us with a call an image, 1292 with one for both, 895 inlined).
+__device__ __forceinline__ void cc_exact_gradients(const float* __restrict__ fimg,
+                                                const float* __restrict__ mimg, const DevGrid& g,
+                                                int x, int y, int z, float gf[3], float gm[3]) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        double a[3], b[3];
+        probe_index(g, x, y, z, d, -1.0, a);
+        probe_index(g, x, y, z, d, +1.0, b);
+        gf[d] = gm[d] = 0.0f;
+        if (!inside_index(a[0], a[1], a[2], g.nx, g.ny, g.nz) ||
+            !inside_index(b[0], b[1], b[2], g.nx, g.ny, g.nz))
+            continue;
+        const int n[3] = {g.nx, g.ny, g.nz};
+        int ia[3], ib[3];
+        float wa[3], wb[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            lin_axis(a[r], n[r], ia[r], wa[r]);
+            lin_axis(b[r], n[r], ib[r], wb[r]);
+        }
+        auto diff = [&](const float* img) {
+            const float v1 = lin_at_axes(img, g.nx, g.ny, ia[0], wa[0], ia[1], wa[1], ia[2], wa[2]);
+            const float v2 = lin_at_axes(img, g.nx, g.ny, ib[0], wb[0], ib[1], wb[1], ib[2], wb[2]);
+            return (float)((double)(v2 - v1) / g.sp[d]);
+        };
+        gf[d] = diff(fimg);
+        gm[d] = diff(mimg);
+    }
 }
 
 // Whether a probe of voxel (x, y, z) along physical axis d is outside the buffer along index axis r,
@@ -210,8 +239,8 @@ __device__ __noinline__ bool cc_probe_outside(const DevGrid& g, int x, int y, in
 
 // One tile (bx, by, bz) of the CC pair: writes the tile's derivative voxels and leaves the
 // thread's sums [cc, |dF|^2, |dM|^2, valid voxels] in acc_out. MODE: how the central differences
-// are formed, ANY grid's, or one of the two usual kinds alone (registers that the other kinds need
-// would be spilled for in the loop).
+// are formed, one kind of grid alone (registers that other kinds need would be spilled for in the
+// loop).
 template <int R, int TY, bool MK, int MODE, class Acc = SumF64>
 __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
                                         unsigned char* smem, const float* __restrict__ fimg,
@@ -365,7 +394,7 @@ __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
     // identity grids: whether the probes of the faces are inside (a coordinate's probes do not
     // depend on the others): bit 0 x, bits 1 and 2 the first and last slice, bit 3 y
     unsigned int ok = ~0u;
-    if ((MODE == CC_AXES || (MODE == CC_ANY && a.identity_dir)) && own) {
+    if ((MODE == CC_AXES || MODE == CC_AXES64) && own) {
         auto inside = [&](int i, int j, int k, int d, int n) {
             return axis_probe_inside(a.g, i, j, k, d, -1.0, n) && axis_probe_inside(a.g, i, j, k, d, +1.0, n);
         };
@@ -526,7 +555,7 @@ __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
         acc_cc += cc;
         // gradients of moving (for the first direction) and of fixed (for the second)
         float gm[3], gf[3];
-        if (MODE == CC_AXES || (MODE == CC_ANY && a.identity_dir)) {
+        if (MODE == CC_AXES || MODE == CC_AXES64) {
             // interp.rs:96-120 on an identity-direction grid: the probes at +-half a spacing lerp
             // halfway toward the neighbours along the axis. Upper probe at p + 0.5: lerp to p + 1
             // unless p is the last voxel; lower probe at p - 0.5: base p - 1 with weight 0.5, or
@@ -580,8 +609,7 @@ __device__ __forceinline__ void cc_tile(const CcArgs& a, int bx, int by, int bz,
                 }
             }
         } else {
-            cc_exact_gradient(mimg, a.g, x, y, z, gm);
-            cc_exact_gradient(fimg, a.g, x, y, z, gf);
+            cc_exact_gradients(fimg, mimg, a.g, x, y, z, gf, gm);
         }
         const float fcf = (float)cf, fcm = (float)cm;
         float dfx = fcf * gm[0], dfy = fcf * gm[1], dfz = fcf * gm[2];
@@ -768,19 +796,15 @@ int launch_radius(fw_ctx* ctx, const CcArgs& a, int radius, const float* f, cons
     case RR:                                                                                    \
         if constexpr (!MK)                                                                      \
             if (c32)                                                                            \
-                return a.mode == CC_ROTATED                                                     \
-                           ? launch_r<RR, CC_TY, false, CC_ROTATED, SumC32>(                    \
-                                 ctx, a, f, m, v, df, dm, d_result, want_norms)                 \
-                           : launch_r<RR, CC_TY, false, CC_ANY, SumC32>(ctx, a, f, m, v, df,    \
-                                                                        dm, d_result,           \
-                                                                        want_norms);            \
-        if (a.mode == CC_AXES)                                                                  \
-            return launch_r<RR, CC_TY, MK, CC_AXES>(ctx, a, f, m, v, df, dm, d_result,          \
-                                                    want_norms);                                \
-        if (a.mode == CC_ROTATED)                                                               \
-            return launch_r<RR, CC_TY, MK, CC_ROTATED>(ctx, a, f, m, v, df, dm, d_result,       \
-                                                       want_norms);                             \
-        return launch_r<RR, CC_TY, MK, CC_ANY>(ctx, a, f, m, v, df, dm, d_result, want_norms);
+                return (a.mode == CC_EXACT     ? launch_r<RR, CC_TY, false, CC_EXACT, SumC32>   \
+                        : a.mode == CC_ROTATED ? launch_r<RR, CC_TY, false, CC_ROTATED, SumC32> \
+                                               : launch_r<RR, CC_TY, false, CC_AXES64, SumC32>)(\
+                    ctx, a, f, m, v, df, dm, d_result, want_norms);                             \
+        return (a.mode == CC_AXES      ? launch_r<RR, CC_TY, MK, CC_AXES>                       \
+                : a.mode == CC_AXES64  ? launch_r<RR, CC_TY, MK, CC_AXES64>                     \
+                : a.mode == CC_ROTATED ? launch_r<RR, CC_TY, MK, CC_ROTATED>                    \
+                                       : launch_r<RR, CC_TY, MK, CC_EXACT>)(                    \
+            ctx, a, f, m, v, df, dm, d_result, want_norms);
     switch (radius) {
         FW_CC_RADIUS(1)
         FW_CC_RADIUS(2)
@@ -834,13 +858,13 @@ CcArgs cc_args(const HostGrid& g, long long ps) {
         a.isp[d] = 1.0 / g.sp[d];
         a.ispf[d] = (float)a.isp[d];
     }
-    a.identity_dir = 1;
+    bool identity = true;
     for (int r = 0; r < 3; ++r)
         for (int c = 0; c < 3; ++c)
-            if (g.dir[r * 3 + c] != (r == c ? 1.0 : 0.0)) a.identity_dir = 0;
+            if (g.dir[r * 3 + c] != (r == c ? 1.0 : 0.0)) identity = false;
     const bool exact = (double)a.ispf[0] == a.isp[0] && (double)a.ispf[1] == a.isp[1] &&
                        (double)a.ispf[2] == a.isp[2];
-    bool stencil = !a.identity_dir;
+    bool stencil = !identity;
     // How far rounding can move a probe's index: a few float64 units of the largest coordinate in
     // voxels (and no less than 1e-9).
     double reach = 0.0, least = g.sp[0];
@@ -887,7 +911,7 @@ CcArgs cc_args(const HostGrid& g, long long ps) {
                 a.weight[p][r] = (float)w;
             }
         }
-    a.mode = a.identity_dir ? (exact ? CC_AXES : CC_ANY) : (stencil ? CC_ROTATED : CC_ANY);
+    a.mode = identity ? (exact ? CC_AXES : CC_AXES64) : (stencil ? CC_ROTATED : CC_EXACT);
     return a;
 }
 
@@ -924,8 +948,9 @@ int launch_cc_pair_batch(fw_ctx* ctx, const HostGrid& g, long long ps, int radiu
 #define FW_CC_BATCH(RR)                                                                          \
     case RR:                                                                                    \
         return (a.mode == CC_AXES      ? launch_cc_batch_r<RR, CC_AXES>                         \
+                : a.mode == CC_AXES64  ? launch_cc_batch_r<RR, CC_AXES64>                       \
                 : a.mode == CC_ROTATED ? launch_cc_batch_r<RR, CC_ROTATED>                      \
-                                       : launch_cc_batch_r<RR, CC_ANY>)(                        \
+                                       : launch_cc_batch_r<RR, CC_EXACT>)(                      \
             ctx, a, L, blocks, fimg, mimg, img_stride, d_fixed, d_moving, field_stride,         \
             partials, part_stride, counter, result, result_stride, want_norms);
     switch (radius) {
@@ -1144,8 +1169,9 @@ extern "C" int fw_cc_value_derivative_pair_noalloc(const fw_grid* grid, const fl
 #define FW_CC_NOALLOC(RR)                                                                        \
     case RR:                                                                                    \
         return (a.mode == CC_AXES      ? noalloc_launch<RR, CC_TY, CC_AXES>                     \
+                : a.mode == CC_AXES64  ? noalloc_launch<RR, CC_TY, CC_AXES64>                   \
                 : a.mode == CC_ROTATED ? noalloc_launch<RR, CC_TY, CC_ROTATED>                  \
-                                       : noalloc_launch<RR, CC_TY, CC_ANY>)(                    \
+                                       : noalloc_launch<RR, CC_TY, CC_EXACT>)(                  \
             a, num_sms, fixed, moving, d_fixed, d_moving, result, s, st);
     switch (radius) {
         FW_CC_NOALLOC(1)
