@@ -111,6 +111,12 @@ struct SmoothArgs {
     float tx_[MAX_TAPS], ty_[MAX_TAPS], tz_[MAX_TAPS];
 };
 
+// A warp's largest |u/sp| (warp_max_f) into the field's: a NaN wins there too, so that a field that is
+// not finite is seen as such (field_ops.rs:191-203).
+__device__ __forceinline__ void publish_max(unsigned int* max_bits, float vmax) {
+    if (vmax > 0.0f || isnan(vmax)) atomicMax(max_bits, __float_as_uint(vmax));
+}
+
 __global__ void __launch_bounds__(SNT) k_smooth(SmoothArgs a, const float* __restrict__ in,
                                                 float* __restrict__ out,
                                                 unsigned int* __restrict__ max_bits) {
@@ -192,7 +198,7 @@ __global__ void __launch_bounds__(SNT) k_smooth(SmoothArgs a, const float* __res
     }
     if (max_bits) {
         vmax = warp_max_f(vmax);
-        if ((tid & 31) == 0 && vmax > 0.0f) atomicMax(max_bits, __float_as_uint(vmax));
+        if ((tid & 31) == 0) publish_max(max_bits, vmax);
     }
 }
 
@@ -409,7 +415,7 @@ __global__ void __launch_bounds__(256, R <= 6 ? 3 : 2) k_smooth_z(SmoothArgs a, 
                                   max_bits != nullptr);
     if (max_bits) {
         vmax = warp_max_f(vmax);
-        if ((threadIdx.x & 31) == 0 && vmax > 0.0f) atomicMax(max_bits, __float_as_uint(vmax));
+        if ((threadIdx.x & 31) == 0) publish_max(max_bits, vmax);
     }
 }
 
@@ -423,7 +429,7 @@ __global__ void __launch_bounds__(256, R <= 6 ? 3 : 2) k_smooth_z_pair(
     float vmax = smooth_z_tile<R>(a, (int)blockIdx.x - side * gz, blockIdx.y, blockIdx.z, p.in[side],
                                   a.ps_out, p.out[side], p.out[side], true);
     vmax = warp_max_f(vmax);
-    if ((threadIdx.x & 31) == 0 && vmax > 0.0f) atomicMax(max_bits + side, __float_as_uint(vmax));
+    if ((threadIdx.x & 31) == 0) publish_max(max_bits + side, vmax);
 }
 
 // The z pass of every active subject of a batch: tmp / in / out at + b * stride, the max of
@@ -444,8 +450,7 @@ __global__ void __launch_bounds__(256) k_smooth_z_batch(SmoothArgs a, BatchList 
         float vmax = smooth_z_tile<R>(a, zb, xb, yb, tmp + b * stride, a.ps_out, in + b * stride,
                                       out + b * stride, true);
         vmax = warp_max_f(vmax);
-        if ((threadIdx.x & 31) == 0 && vmax > 0.0f)
-            atomicMax(max_bits + b * max_stride, __float_as_uint(vmax));
+        if ((threadIdx.x & 31) == 0) publish_max(max_bits + b * max_stride, vmax);
     }
 }
 

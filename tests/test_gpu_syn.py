@@ -111,6 +111,27 @@ def test_a_step_matches_on_every_route_of_its_two_sides(backend, size, variance,
         assert np.abs(backend.download_field(state[k]) - ostate[k]).max() <= 1e-4
 
 
+@pytest.mark.parametrize("size,variance", [((33, 29, 21), 3.0), ((33, 29, 5), 3.0), ((33, 29, 21), 0.0),
+                                           ((166, 166, 167), 3.0)])
+def test_a_gradient_that_is_not_finite_is_reported_as_such(backend, size, variance):
+    """A NaN of the update's largest vector wins over the finite ones on every route of the smoothing
+    (both sides together, taps that differ by axis, none, one side after the other)."""
+    from fastwarp_b200 import FastwarpError, make_grid
+    rng = np.random.default_rng(3)
+    g = make_grid(size)
+    f = rng.random(size[::-1], np.float32)
+    m = f[::-1].copy()
+    m[size[2] // 2, 10:13, 12:15] = np.nan
+    r = SynRecipe(gradient_step=0.25, update_field_variance=variance, cc_radius=2, iterations=[1],
+                  shrink_factors=[1], smoothing_sigmas=[0.0], convergence_threshold=-1.0)
+    fi, mi = backend.upload_image(g, f), backend.upload_image(g, m)
+    state = {k: backend.zero_field(g) for k in ("f2m", "f2m_inv", "m2m", "m2m_inv")}
+    with pytest.raises(FastwarpError, match="the metric gradient is not finite"):
+        syn_step(backend, r, [fi], [mi], None, state, want_updates=False)
+    for b in (fi, mi, *state.values()):
+        b.free()
+
+
 def test_full_registration_matches_the_oracle(backend, pair):
     g, fixed, moving = pair
     r = config1(30)
