@@ -712,13 +712,15 @@ int syn_run_device(fw_ctx* ctx, const fw_syn_recipe* r, const fw_image* const* f
     }
     int total_iters = 0;
     for (int l = 0; l < r->levels; ++l) total_iters += (int)r->iterations[l];
-    // scratch for every reduction of the biggest level, before any capture
-    {
-        HostGrid last;
-        FW_TRY(level_grid(r, fg, r->levels - 1, last));
-        FW_TRY(ensure_scratch(ctx, std::max<size_t>(SLOT_PARTIALS + (size_t)(1 << 20),
-                                                    inv_scratch_doubles(last))));
+    // scratch for every reduction of the biggest level (any of them: shrink factors may grow), before
+    // any capture
+    size_t scratch = SLOT_PARTIALS + (size_t)(1 << 20);
+    for (int l = 0; l < r->levels; ++l) {
+        HostGrid g;
+        FW_TRY(level_grid(r, fg, l, g));
+        scratch = std::max(scratch, inv_scratch_doubles(g));
     }
+    FW_TRY(ensure_scratch(ctx, scratch));
     RunScratch rs;
     FW_TRY(rs.init(ctx, C, std::max(total_iters, 1)));
     FW_TRY(upload_syn_dev(ctx, r, rs.d.syn, fixed_mask || moving_mask));

@@ -132,6 +132,23 @@ def test_a_gradient_that_is_not_finite_is_reported_as_such(backend, size, varian
         b.free()
 
 
+def test_a_first_level_larger_than_the_last_finds_its_scratch():
+    """Shrink factors that grow, on a context of its own: the scratch is sized before the first level's
+    graph is captured, for whichever level is the largest."""
+    from fastwarp_b200 import CudaBackend, make_grid, run_syn_device
+    size = (9, 1200, 1200)  # tiles of 32 columns: more scratch than the million numbers every run has
+    g = make_grid(size)
+    f = np.random.default_rng(3).random(size[::-1], np.float32)
+    r = SynRecipe(gradient_step=0.25, update_field_variance=3.0, cc_radius=2, iterations=[1, 1],
+                  shrink_factors=[1, 2], smoothing_sigmas=[0.0, 0.0], convergence_threshold=-1.0)
+    with CudaBackend(0) as b:
+        fi, mi = b.upload_image(g, f), b.upload_image(g, f[:, :, ::-1].copy())
+        w, iw, recs = run_syn_device(b, r, [fi], [mi])
+        assert [q["level"] for q in recs] == [0, 1]
+        for q in (fi, mi, w, iw):
+            q.free()
+
+
 def test_full_registration_matches_the_oracle(backend, pair):
     g, fixed, moving = pair
     r = config1(30)
