@@ -825,8 +825,9 @@ __global__ void __launch_bounds__(MI_THREADS) k_dense_deriv(
     const DenseState S = *st;
     const int nx = a.g.nx, ny = a.g.ny, nz = a.g.nz;
     double n0 = 0.0, n1 = 0.0;
-    int x, y, z0, z1;
-    if (column_of(nx, ny, nz, a.zchunk, x, y, z0, z1)) {
+    int bx, by, bz, x, y, z0, z1;
+    tile_coords((int)blockIdx.x, (nx + 31) / 32, (ny + 7) / 8, bx, by, bz);
+    if (column_of_tile(nx, ny, nz, a.zchunk, bx, by, bz, x, y, z0, z1)) {
         const int sxy = nx * ny;
         const int col = y * nx + x;
         // identity grids: whether each face probe is inside, and the neighbours' offsets
@@ -865,7 +866,7 @@ __global__ void __launch_bounds__(MI_THREADS) k_dense_deriv(
                 float gm[3], gf[3];
                 if (IDENTITY) {
                     // interp.rs:96-120 at +-half a spacing: halfway to the neighbours
-                    // (central_difference_voxel's arithmetic)
+                    // (the face probes decided by axis_probe_inside)
                     auto diff = [&](int d, bool ok, bool has_lo, bool has_hi, float2 p, float2 q) {
                         const float f2 = has_hi ? fmaf(q.x - cur.x, 0.5f, cur.x) : cur.x;
                         const float f1 = has_lo ? fmaf(cur.x - p.x, 0.5f, p.x) : cur.x;
@@ -907,12 +908,11 @@ __global__ void __launch_bounds__(MI_THREADS) k_dense_deriv(
         red[1][threadIdx.x >> 5] = n1;
     }
     __syncthreads();
-    const unsigned int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    const unsigned int nblocks = gridDim.x * gridDim.y * gridDim.z;
+    const unsigned int nblocks = gridDim.x;
     if (threadIdx.x < 2) {
         double s = 0.0;
         for (int w = 0; w < MI_THREADS / 32; ++w) s += red[threadIdx.x][w];
-        partials[(size_t)bid * 2 + threadIdx.x] = s;
+        partials[(size_t)blockIdx.x * 2 + threadIdx.x] = s;
     }
     if (!mi_last_block(counter, nblocks)) return;
     __shared__ double fin[MI_THREADS / 32];
@@ -1440,13 +1440,14 @@ std::string empty_range_message(const char* role, bool masked) {
     return std::string("the ") + role + " image has no finite voxel";
 }
 
-// The gradient pass's grid on `g`: 32 x 8 columns, z chunks for about eight blocks an SM (every
-// block loads the two ratio tables first, 16 KB).
-dim3 dense_deriv_grid(const HostGrid& g, int num_sms, int* zchunk) {
+// The gradient pass's blocks on `g`: 32 x 8 columns, z chunks for about eight blocks an SM (every
+// block loads the two ratio tables first, 16 KB). In one dimension: an axis takes up to 2^20 voxels,
+// more rows of tiles than the second dimension of a launch.
+unsigned int dense_deriv_blocks(const HostGrid& g, int num_sms, int* zchunk) {
     const long long gx = (g.n[0] + 31) / 32, gy = (g.n[1] + 7) / 8;
     const long long want = std::max<long long>(1, (8LL * num_sms + gx * gy - 1) / (gx * gy));
     *zchunk = (int)std::max<long long>(1, (g.n[2] + want - 1) / want);
-    return dim3((unsigned int)gx, (unsigned int)gy, (unsigned int)((g.n[2] + *zchunk - 1) / *zchunk));
+    return (unsigned int)(gx * gy * ((g.n[2] + *zchunk - 1) / *zchunk));
 }
 
 }  // namespace
@@ -1477,11 +1478,11 @@ int dense_mi_create(fw_ctx* ctx, int bins, const HostGrid& g, fw_dense_mi** out)
     d->ctx = ctx;
     d->bins = bins;
     int zchunk = 1;
-    const dim3 dg = dense_deriv_grid(g, ctx->num_sms, &zchunk);
+    const size_t blocks = dense_deriv_blocks(g, ctx->num_sms, &zchunk);
     const size_t cells = (size_t)bins * bins + bins;
     const size_t o_hist = 512, o_ratio = o_hist + 16 * cells,
                  o_part = o_ratio + 16 * (size_t)bins * bins;
-    d->bytes = o_part + 16 * (size_t)dg.x * dg.y * dg.z;
+    d->bytes = o_part + 16 * blocks;
     static_assert(sizeof(DenseState) <= 256, "the state's place in the scratch");
     int rc = dev_alloc(ctx, d->bytes, &d->base);
     if (rc) {
@@ -1547,7 +1548,7 @@ int enqueue_dense_mi_pair(fw_ctx* ctx, const fw_image* f, const fw_image* m, con
         for (int c = 0; c < 3; ++c)
             if (g.dir[r * 3 + c] != (r == c ? 1.0 : 0.0)) identity = false;
     for (int d = 0; d < 3; ++d) da.isp[d] = 1.0 / g.sp[d];
-    const dim3 grid = dense_deriv_grid(g, ctx->num_sms, &da.zchunk);
+    const unsigned int grid = dense_deriv_blocks(g, ctx->num_sms, &da.zchunk);
     auto deriv = identity ? k_dense_deriv<true> : k_dense_deriv<false>;
     deriv<<<grid, MI_THREADS, 0, ctx->stream>>>(da, f->d, m->d, fmp, mmp, sc->st, sc->ratio,
                                                 d_fixed->d, d_moving->d, sc->partials, sc->counter,

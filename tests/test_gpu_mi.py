@@ -164,6 +164,25 @@ def test_dense_histogram_merges_its_words_before_they_overflow(backend):
     assert np.allclose(out[0], out[1], rtol=1e-12, atol=0.0)
 
 
+def test_dense_pair_on_an_axis_of_half_a_million_voxels(backend):
+    """More rows of 8 than the second dimension of a launch holds: the pair of the same image with its
+    long axis along x gives the same histograms, and gradients with x and y exchanged."""
+    long, rng = 530000, np.random.default_rng(5)
+    f = rng.random((2, long, 3), np.float32)
+    m = f * f + 0.1 * rng.random(f.shape, np.float32)
+    out = []
+    for a, b in ((f, m), (f.transpose(0, 2, 1), m.transpose(0, 2, 1))):
+        g = make_grid(a.shape[::-1])
+        fi, mi = (backend.upload_image(g, np.ascontiguousarray(v)) for v in (a, b))
+        (v0, d0), (v1, d1) = backend.mi_value_derivative_pair(fi, mi, 32)
+        out.append((v0, v1, backend.download_field(d0), backend.download_field(d1)))
+        for q in (fi, mi, d0, d1):
+            q.free()
+    assert out[0][:2] == out[1][:2]
+    for d, e in zip(out[0][2:], out[1][2:]):
+        assert np.array_equal(d, e.transpose(0, 2, 1, 3)[..., [1, 0, 2]])
+
+
 @pytest.mark.parametrize("where", ["jittered", "centres", "faces"])
 def test_gradient_on_an_axis_aligned_image_matches(backend, where):
     """The gradient from a sample's own corners and four more an axis: inside the image, at voxel
