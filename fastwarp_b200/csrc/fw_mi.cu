@@ -805,12 +805,15 @@ __device__ __forceinline__ void dense_outputs(double w0, double w1, float gm[3],
 // direction), zero where the voxel does not contribute; result[0..1] = their sums of squares, and
 // the last block publishes the pair's scalars.
 //
-// 32 x 8 column tiles marching along z. With IDENTITY (axis-aligned grids) a column keeps its two
-// images' previous, current and next slices in registers, so a voxel loads one new value and the
-// four neighbours of its slice for each image, and decides the face probes of x and y once; a
-// rotated grid takes the exact probes of every voxel. Bound by the f64 spline weights and the
-// eight ratio reads from shared memory. 193 x 229 x 193: 494 us with a voxel a thread over a
-// 296-block grid, 185 us.
+// A thread takes a column and a chunk of z (consecutive threads consecutive columns, whatever the
+// grid's width, then the next chunk) and marches along z. With IDENTITY (an identity direction) a
+// column keeps its two images' previous, current and next slices in registers, so a voxel loads one new
+// value and the four neighbours of its slice for each image, and decides the face probes of x and y
+// once; any other direction takes the exact probes of every voxel. Bound by the f64 spline weights
+// and the eight ratio reads from shared memory. The pair's whole call at 193 x 229 x 193: 1420 us with
+// a voxel a thread over a 296-block grid (the pass 494) and the histogram of 64-bit cells, 336 with
+// columns in tiles of 32 x 8 (the pass 185), 323 now; turned 2120, 1390 and 960. At 1 x 1000 x 1000, where
+// such a tile has one column in 32: 172, 560 and 107 us.
 template <bool IDENTITY>
 __global__ void __launch_bounds__(MI_THREADS) k_dense_deriv(
     DenseArgs a, const float* __restrict__ f, const float* __restrict__ m,
@@ -825,11 +828,12 @@ __global__ void __launch_bounds__(MI_THREADS) k_dense_deriv(
     const DenseState S = *st;
     const int nx = a.g.nx, ny = a.g.ny, nz = a.g.nz;
     double n0 = 0.0, n1 = 0.0;
-    int bx, by, bz, x, y, z0, z1;
-    tile_coords((int)blockIdx.x, (nx + 31) / 32, (ny + 7) / 8, bx, by, bz);
-    if (column_of_tile(nx, ny, nz, a.zchunk, bx, by, bz, x, y, z0, z1)) {
-        const int sxy = nx * ny;
-        const int col = y * nx + x;
+    const int sxy = nx * ny;
+    const long long t = (long long)blockIdx.x * MI_THREADS + threadIdx.x;
+    const long long z0 = t / sxy * a.zchunk;
+    if (z0 < nz) {
+        const int z1 = (int)min(z0 + a.zchunk, (long long)nz);
+        const int col = (int)(t % sxy), y = col / nx, x = col - y * nx;
         // identity grids: whether each face probe is inside, and the neighbours' offsets
         bool okx = true, oky = true;
         float2 lo = make_float2(0.0f, 0.0f), cur = lo, hi = lo;  // (f, m) of slices z - 1, z, z + 1
@@ -844,7 +848,7 @@ __global__ void __launch_bounds__(MI_THREADS) k_dense_deriv(
             if (z0 > 0) lo = at(z0 - 1);
             cur = at(z0);
         }
-        for (int z = z0; z < z1; ++z) {
+        for (int z = (int)z0; z < z1; ++z) {
             const long long l = (long long)z * sxy + col;
             if (IDENTITY) {
                 if (z + 1 < nz) hi = at(z + 1);
@@ -1440,14 +1444,14 @@ std::string empty_range_message(const char* role, bool masked) {
     return std::string("the ") + role + " image has no finite voxel";
 }
 
-// The gradient pass's blocks on `g`: 32 x 8 columns, z chunks for about eight blocks an SM (every
-// block loads the two ratio tables first, 16 KB). In one dimension: an axis takes up to 2^20 voxels,
-// more rows of tiles than the second dimension of a launch.
+// The gradient pass's blocks on `g`: a thread a column and z chunk, the chunks for about eight blocks
+// an SM (every block loads the two ratio tables first, 16 KB).
 unsigned int dense_deriv_blocks(const HostGrid& g, int num_sms, int* zchunk) {
-    const long long gx = (g.n[0] + 31) / 32, gy = (g.n[1] + 7) / 8;
-    const long long want = std::max<long long>(1, (8LL * num_sms + gx * gy - 1) / (gx * gy));
+    const long long cols = g.n[0] * g.n[1];
+    const long long want = (8LL * num_sms * MI_THREADS + cols - 1) / cols;
     *zchunk = (int)std::max<long long>(1, (g.n[2] + want - 1) / want);
-    return (unsigned int)(gx * gy * ((g.n[2] + *zchunk - 1) / *zchunk));
+    const long long chunks = (g.n[2] + *zchunk - 1) / *zchunk;
+    return (unsigned int)((cols * chunks + MI_THREADS - 1) / MI_THREADS);
 }
 
 }  // namespace

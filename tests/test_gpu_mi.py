@@ -270,6 +270,24 @@ def test_dense_mi_pair_matches_the_oracle(backend, bins, oblique):
     assert np.array_equal(backend.download_field(c0), g0)
 
 
+@pytest.mark.parametrize("size", [(1, 40, 37), (2, 31, 33), (33, 3, 40), (40, 41, 1), (257, 5, 9), (1, 1, 300)])
+@pytest.mark.parametrize("turned", [False, True])
+def test_dense_mi_pair_on_thin_grids_matches_the_oracle(backend, size, turned):
+    """Columns of every width: chunks of z and ends of blocks inside a row, an axis of one voxel."""
+    rng = np.random.default_rng(size[0])
+    geo = ((1.0, 1.5, 0.9), (-3.0, 2.0, 1.0), rot_z(0.2) @ rot_x(-0.1) if turned else np.eye(3))
+    og, g = O.make_grid(size, *geo), make_grid(size, *geo)
+    f = rng.random(size[::-1], np.float32)
+    m = (f * f + 0.1 * rng.random(f.shape, np.float32)).astype(np.float32)
+    fi, mi = backend.upload_image(g, f), backend.upload_image(g, m)
+    ((v0, d0), (v1, d1)), norms = backend.mi_value_derivative_pair_with_norms(fi, mi, 32)
+    (w0, _, e0), (w1, _, e1) = oracle_pair(og, f, m, 32)
+    assert abs(v0 - w0) <= 1e-5 * abs(w0) and abs(v1 - w1) <= 1e-5 * abs(w1)
+    for d, e, n in ((d0, e0, norms[0]), (d1, e1, norms[1])):
+        assert np.abs(backend.download_field(d) - e).max() <= 5e-4 * np.abs(e).max()
+        assert abs(n - np.sqrt((e ** 2).sum())) <= 5e-4 * np.sqrt((e ** 2).sum())
+
+
 def test_masked_dense_mi_pair_matches_the_oracle(backend):
     og, g, f, m = dense_case(seed=9)
     nz, ny, nx = f.shape
