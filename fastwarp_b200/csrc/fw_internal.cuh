@@ -533,10 +533,9 @@ struct InvState {
 // The inversion loop (fw_invert.cu). `res` (a field on the inverse's grid) keeps the residual
 // of the last measurement for the body that follows.
 int enqueue_inversion_prefix(fw_ctx* ctx, const fw_field* field, fw_field* inverse,
-                             fw_field* res, const fw_invert_params& prm, InvState* st,
-                             cudaGraphConditionalHandle handle, int use_handle);
+                             fw_field* res, const fw_invert_params& prm, InvState* st);
 int enqueue_inversion_body(fw_ctx* ctx, const fw_field* field, fw_field* inverse, fw_field* res,
-                           InvState* st, cudaGraphConditionalHandle handle, int use_handle);
+                           InvState* st);
 // One body of the same inversion of both sides of a SyN iteration in one launch of each kernel:
 // inverse[s] against field[s] with the state st[2 s]; a side whose loop has ended does nothing. With
 // use_handle the condition is set to whether either side runs another body.
@@ -703,7 +702,7 @@ enum Slot : int {
     SLOT_NORM_A = 3,     // sum u.u of derivative a
     SLOT_NORM_B = 4,
     SLOT_CC_VALID = 5,   // valid voxels of the masked CC
-    SLOT_INV = 8,        // inversion state (8 doubles)
+    SLOT_INV = 8,        // inversion state (InvState)
     SLOT_MI = 32,        // MI scalars
     SLOT_PARTIALS = 128, // block partials follow
 };

@@ -169,15 +169,12 @@ __device__ __forceinline__ void init_state(InvState* __restrict__ st, const fw_i
     st->run = 0;
 }
 
-__global__ void k_inv_init(InvState* __restrict__ st, fw_invert_params prm,
-                           cudaGraphConditionalHandle handle, int use_handle) {
-    init_state(st, prm);
-    if (use_handle) cudaGraphSetConditional(handle, st->go ? 1u : 0u);
-}
+__global__ void k_inv_init(InvState* __restrict__ st, fw_invert_params prm) { init_state(st, prm); }
 
 // Several inversions' settings in one launch: states st[0..count), and the conditions of the WHILE
-// nodes hs.h[0..nhandles) cleared (the bodies ahead of a node set it); it also clears zero[0..nzero) (the SyN level graph begins every iteration
-// with it: its four inversions' settings, its two loops and the update maxima, in one node).
+// nodes hs.h[0..nhandles) cleared (the bodies ahead of a node set it); it also clears zero[0..nzero)
+// (the SyN level graph begins every iteration with it: its four inversions' settings, its two loops
+// and the update maxima, in one node).
 struct InitHandles {
     cudaGraphConditionalHandle h[kMaxInitHandles];
 };
@@ -347,7 +344,7 @@ __device__ __forceinline__ void step_block(const InvArgs& a, int bx, int by, int
 
 // The last block's record of body k (field_ops.rs:339-355): errors, bodies executed, the step
 // and clamp the fix kernel applies, and whether body k + 1 runs.
-__device__ __forceinline__ bool finish_step(InvState* __restrict__ st, double s, double m,
+__device__ __forceinline__ void finish_step(InvState* __restrict__ st, double s, double m,
                                             double count) {
     const int kb = st->k;
     const float eps = kb == 0 ? 0.75f : 0.5f;
@@ -361,7 +358,6 @@ __device__ __forceinline__ bool finish_step(InvState* __restrict__ st, double s,
     st->limit = eps * (float)m;
     st->lb = 0u;
     st->go = next ? 1 : 0;
-    return next;
 }
 
 // Body k of the loop: measurement of psi against f (its mean and max), the update of every tile
@@ -374,25 +370,16 @@ __global__ void __launch_bounds__(256, FW_STEP_MIN_BLOCKS) k_inv_step(InvArgs a,
                                                      double* __restrict__ partials,
                                                      unsigned int* __restrict__ counter,
                                                      InvState* __restrict__ st,
-                                                     unsigned int* __restrict__ defer,
-                                                     cudaGraphConditionalHandle handle,
-                                                     int use_handle) {
+                                                     unsigned int* __restrict__ defer) {
     pdl_wait();
-    if (!st->go) {  // uniform: the state only changes in the last block of a working grid
-        if (use_handle && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 &&
-            threadIdx.x == 0)
-            cudaGraphSetConditional(handle, 0u);
-        return;
-    }
+    if (!st->go) return;  // uniform: the state only changes in the last block of a working grid
     double sum = 0.0;
     float mx = 0.0f;
     step_block(a, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, f, psi, res, st, defer, sum, mx);
     const unsigned int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     const unsigned int nblocks = gridDim.x * gridDim.y * gridDim.z;
-    reduce_and_finish(sum, mx, partials, counter, bid, nblocks, [&](double s, double m) {
-        const bool next = finish_step(st, s, m, (double)a.g.n);
-        if (use_handle) cudaGraphSetConditional(handle, next ? 1u : 0u);
-    });
+    reduce_and_finish(sum, mx, partials, counter, bid, nblocks,
+                      [&](double s, double m) { finish_step(st, s, m, (double)a.g.n); });
 }
 
 // The deferred warp parts of the body that just ran, entries vb * 8 + w, + 8 nvb, ... of the list
@@ -634,15 +621,13 @@ static unsigned int* defer_list(fw_ctx* ctx, const HostGrid& g) {
     return reinterpret_cast<unsigned int*>(ctx->d_scratch + SLOT_PARTIALS + 2 * inv_step_tiles(g));
 }
 
-// Before the loop: scratch for its bodies and the loop's settings (the init kernel also sets the
-// WHILE node's condition in graph mode).
+// Before the loop: scratch for its bodies and the loop's settings.
 int enqueue_inversion_prefix(fw_ctx* ctx, const fw_field* field, fw_field* inverse,
-                             fw_field* res, const fw_invert_params& prm, InvState* st,
-                             cudaGraphConditionalHandle handle, int use_handle) {
+                             fw_field* res, const fw_invert_params& prm, InvState* st) {
     FW_CHECK(res->grid.same(inverse->grid) && res->ps == inverse->ps,
              "invert: the residual buffer does not match the inverse");
     FW_TRY(ensure_scratch(ctx, inv_scratch_doubles(field->grid)));
-    k_inv_init<<<1, 1, 0, ctx->stream>>>(st, prm, handle, use_handle);
+    k_inv_init<<<1, 1, 0, ctx->stream>>>(st, prm);
     return check_launch(ctx, "k_inv_init");
 }
 
@@ -666,8 +651,7 @@ int enqueue_inversion_inits(fw_ctx* ctx, InvState* st, int count, const fw_inver
 
 // One kernel of a body: 0 bound, 1 step, 2 fix (each returns at once when the loop has ended).
 static int launch_body_kernel(fw_ctx* ctx, const fw_field* field, fw_field* inverse,
-                              fw_field* res, InvState* st, int which,
-                              cudaGraphConditionalHandle handle, int use_handle) {
+                              fw_field* res, InvState* st, int which) {
     InvArgs a = inv_args(field, inverse);
     const dim3 g = step_grid(ctx, a);
     unsigned int* defer = defer_list(ctx, field->grid);
@@ -681,8 +665,7 @@ static int launch_body_kernel(fw_ctx* ctx, const fw_field* field, fw_field* inve
     if (which == 1)
         return launch_pdl(ctx, "k_inv_step", k_inv_step, g, dim3(256), 0, a,
                           (const float*)field->d, inverse->d, res->d,
-                          ctx->d_scratch + SLOT_PARTIALS, ctx->d_counter + 2, st, defer, handle,
-                          use_handle);
+                          ctx->d_scratch + SLOT_PARTIALS, ctx->d_counter + 2, st, defer);
     const unsigned int tiles = (unsigned int)inv_step_tiles(field->grid);
     const unsigned int nf = std::max(1u, std::min(tiles, 2u * (unsigned int)ctx->num_sms));
     return launch_pdl(ctx, "k_inv_fix", k_inv_fix, dim3(nf), dim3(256), 0, a, inverse->d,
@@ -691,15 +674,15 @@ static int launch_body_kernel(fw_ctx* ctx, const fw_field* field, fw_field* inve
 
 // One body: bound, step, fix.
 int enqueue_inversion_body(fw_ctx* ctx, const fw_field* field, fw_field* inverse, fw_field* res,
-                           InvState* st, cudaGraphConditionalHandle handle, int use_handle) {
+                           InvState* st) {
     for (int which = 0; which < 3; ++which)
-        FW_TRY(launch_body_kernel(ctx, field, inverse, res, st, which, handle, use_handle));
+        FW_TRY(launch_body_kernel(ctx, field, inverse, res, st, which));
     return 0;
 }
 
 int enqueue_inversion_kernel(fw_ctx* ctx, const fw_field* field, fw_field* inverse, fw_field* res,
                              InvState* st, int which) {
-    return launch_body_kernel(ctx, field, inverse, res, st, which, 0, 0);
+    return launch_body_kernel(ctx, field, inverse, res, st, which);
 }
 
 // One inversion's scratch: its step's partials, then its deferred list (even, so that the next
@@ -824,11 +807,11 @@ int invert_field(fw_ctx* ctx, const fw_field* field, fw_field* inverse,
         fw_field* f;
         ~Free() { fw_field_free(f); }
     } guard{res};
-    FW_TRY(enqueue_inversion_prefix(ctx, field, inverse, res, prm, st, 0, 0));
+    FW_TRY(enqueue_inversion_prefix(ctx, field, inverse, res, prm, st));
     InvState h{};
     if (prm.max_iterations <= 0) FW_TRY(sync(ctx));
     for (int body = 0; body < prm.max_iterations; ++body) {
-        FW_TRY(enqueue_inversion_body(ctx, field, inverse, res, st, 0, 0));
+        FW_TRY(enqueue_inversion_body(ctx, field, inverse, res, st));
         FW_CUDA(cudaMemcpyAsync(ctx->h_pinned, st, sizeof(InvState), cudaMemcpyDeviceToHost,
                                 ctx->stream));
         FW_TRY(sync(ctx));  // the state that ends the loop is the one it reports
@@ -839,16 +822,6 @@ int invert_field(fw_ctx* ctx, const fw_field* field, fw_field* inverse,
     stats->mean_error_norm = h.executed == 0 ? 0.0 : h.mean;
     stats->max_error_norm = h.executed == 0 ? 0.0 : h.max;
     return 0;
-}
-
-size_t inv_state_bytes() { return sizeof(InvState); }
-
-void inv_state_read(const void* raw, fw_invert_stats* stats) {
-    InvState h;
-    std::memcpy(&h, raw, sizeof(h));
-    stats->iterations = h.executed;
-    stats->mean_error_norm = h.executed == 0 ? 0.0 : h.mean;
-    stats->max_error_norm = h.executed == 0 ? 0.0 : h.max;
 }
 
 }  // namespace fw

@@ -77,19 +77,19 @@ int fw_time_kernels(fw_ctx* ctx, const fw_image* fixed, const fw_image* moving, 
                 case 2: return launch_smooth(ctx, a, s, variance, bits, e);
                 case 3: return launch_compose(ctx, u, w, w, bits, 0.1);
                 case 4: {  // a first body of a fresh loop from a zero inverse
-                    FW_TRY(enqueue_inversion_prefix(ctx, u, w, e, once, st, 0, 0));
-                    return enqueue_inversion_body(ctx, u, w, e, st, 0, 0);
+                    FW_TRY(enqueue_inversion_prefix(ctx, u, w, e, once, st));
+                    return enqueue_inversion_body(ctx, u, w, e, st);
                 }
                 case 5: return enqueue_inversion_kernel(ctx, u, w, e, st, 0);
                 case 6: return enqueue_inversion_kernel(ctx, u, w, e, st, 2);
-                default: return enqueue_inversion_prefix(ctx, u, w, e, once, st, 0, 0);
+                default: return enqueue_inversion_prefix(ctx, u, w, e, once, st);
             }
         };
         if (kind == 4 || kind == 5 || kind == 6) {  // every timed body starts from psi = 0
             FW_CUDA(cudaMemsetAsync(w->d, 0, w->bytes, ctx->stream));
         }
         if (kind == 5 || kind == 6) {  // a loop before its first body (and after its step)
-            rc = enqueue_inversion_prefix(ctx, u, w, e, once, st, 0, 0);
+            rc = enqueue_inversion_prefix(ctx, u, w, e, once, st);
             if (!rc && kind == 6) rc = enqueue_inversion_kernel(ctx, u, w, e, st, 0);
             if (!rc && kind == 6) rc = enqueue_inversion_kernel(ctx, u, w, e, st, 1);
             if (rc) break;
