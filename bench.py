@@ -83,8 +83,8 @@ def parse():
 
 
 def time_kernels(b, fimg, mimg, reps):
-    """Per-kernel mean ms and algorithmic bytes at the grid of the images (CUDA events on the
-    engine's stream)."""
+    """Mean ms and algorithmic bytes of a SyN iteration's steps, both sides, at the grid of the images
+    (CUDA events on the engine's stream)."""
     import ctypes as C
 
     from fastwarp_b200 import _native as N
@@ -369,9 +369,9 @@ def run_ours(args, rank, world, local):
     # per-kernel roofline at the finest level (CUDA events on the engine stream)
     log("kernel timing")
     t = time_kernels(b, fi, b.upload_image(g, fixed), 20)
-    # launches per iteration (ncu launch list of a registration: 4 inversions of 1.08 bodies on
-    # average, each body its bound, step and fix kernels; the step carries the body's bytes)
-    per_iter = {"warp": 2, "cc_pair": 1, "smooth": 2, "compose": 2, "inv_step": 4.3}
+    # runs per iteration (ncu launch list of a registration: 2 inversions of both sides, of 1.08
+    # bodies on average, each body its bound, step and fix kernels; the step carries the body's bytes)
+    per_iter = {"warp": 1, "cc_pair": 1, "smooth": 1, "compose": 1, "inv_step": 2.15}
     dom = max(per_iter, key=lambda k: t[k][0] * per_iter[k])
     ms, by = t[dom]
     peak, src = peaks()

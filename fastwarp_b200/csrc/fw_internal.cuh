@@ -538,10 +538,11 @@ int enqueue_inversion_body(fw_ctx* ctx, const fw_field* field, fw_field* inverse
                            InvState* st);
 // One body of the same inversion of both sides of a SyN iteration in one launch of each kernel:
 // inverse[s] against field[s] with the state st[2 s]; a side whose loop has ended does nothing. With
-// use_handle the condition is set to whether either side runs another body.
+// use_handle the condition is set to whether either side runs another body. `which`: one of its
+// kernels alone (0 bound, 1 step, 2 fix), for kernel timing.
 int enqueue_inversion_pair_body(fw_ctx* ctx, const fw_field* const field[2],
                                 fw_field* const inverse[2], fw_field* const res[2], InvState* st,
-                                cudaGraphConditionalHandle handle, int use_handle);
+                                cudaGraphConditionalHandle handle, int use_handle, int which = -1);
 int enqueue_inversion_pair_init(fw_ctx* ctx, const fw_invert_params& prm, InvState* st);
 // Graph mode: scratch for an inversion's bodies without the init kernel, and the inits of an
 // iteration's inversions (their states and up to kMaxInitHandles WHILE conditions) in one kernel that
@@ -551,9 +552,6 @@ int inversion_scratch(fw_ctx* ctx, const fw_field* field);
 int enqueue_inversion_inits(fw_ctx* ctx, InvState* st, int count, const fw_invert_params& prm,
                             const cudaGraphConditionalHandle* handles, int nhandles,
                             unsigned int* zero, int nzero);
-// One kernel of a body (0 bound, 1 step, 2 fix), for kernel timing.
-int enqueue_inversion_kernel(fw_ctx* ctx, const fw_field* field, fw_field* inverse, fw_field* res,
-                             InvState* st, int which);
 long long inv_step_tiles(const HostGrid& g);
 // Warp parts of the step's tiles on grid g (the capacity of a deferred list).
 long long inv_step_parts(const HostGrid& g);
@@ -676,6 +674,9 @@ int batch_syn_run(fw_ctx* ctx, const fw_syn_recipe* r, const fw_image* const* fi
                   const fw_batch_subject* subj, fw_field** warps, fw_field** inverses,
                   fw_syn_iteration* records, int64_t cap, int64_t* counts, int32_t* statuses,
                   fw_batch_report* report);
+
+// How many sides one launch of an iteration's smoothing and composition takes (fw_syn.cu).
+int syn_sides_together(const HostGrid& g);
 
 // The SyN stage on device images (fw_syn.cu); masks may be null; prior / prior_inverse are the
 // earlier SyN stages' collapsed fields (both null for a first stage).

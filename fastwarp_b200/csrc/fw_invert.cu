@@ -680,11 +680,6 @@ int enqueue_inversion_body(fw_ctx* ctx, const fw_field* field, fw_field* inverse
     return 0;
 }
 
-int enqueue_inversion_kernel(fw_ctx* ctx, const fw_field* field, fw_field* inverse, fw_field* res,
-                             InvState* st, int which) {
-    return launch_body_kernel(ctx, field, inverse, res, st, which);
-}
-
 // One inversion's scratch: its step's partials, then its deferred list (even, so that the next
 // one's partials stay aligned).
 static size_t inv_side_doubles(const HostGrid& g) {
@@ -703,7 +698,7 @@ int enqueue_inversion_pair_init(fw_ctx* ctx, const fw_invert_params& prm, InvSta
 
 int enqueue_inversion_pair_body(fw_ctx* ctx, const fw_field* const field[2],
                                 fw_field* const inverse[2], fw_field* const res[2], InvState* st,
-                                cudaGraphConditionalHandle handle, int use_handle) {
+                                cudaGraphConditionalHandle handle, int use_handle, int which) {
     InvPair p;
     p.a = inv_args(field[0], inverse[0]);
     const dim3 g = step_grid(ctx, p.a);
@@ -723,9 +718,12 @@ int enqueue_inversion_pair_body(fw_ctx* ctx, const fw_field* const field[2],
     const Lattice t = lattice_of(p.a.g);
     const unsigned int nb = (unsigned int)std::max<long long>(
         1, std::min<long long>((t.count() + 255) / 256, 4LL * ctx->num_sms));
-    FW_TRY(launch_pdl(ctx, "k_inv_bound_pair", k_inv_bound_pair, dim3(nb, 2), dim3(256), 0, p, t));
-    FW_TRY(launch_pdl(ctx, "k_inv_step_pair", k_inv_step_pair, dim3(2 * g.x, g.y, g.z), dim3(256), 0,
-                      p, (int)g.x, handle, use_handle));
+    if (which < 0 || which == 0)
+        FW_TRY(launch_pdl(ctx, "k_inv_bound_pair", k_inv_bound_pair, dim3(nb, 2), dim3(256), 0, p, t));
+    if (which < 0 || which == 1)
+        FW_TRY(launch_pdl(ctx, "k_inv_step_pair", k_inv_step_pair, dim3(2 * g.x, g.y, g.z), dim3(256),
+                          0, p, (int)g.x, handle, use_handle));
+    if (which >= 0 && which != 2) return 0;
     const unsigned int tiles = (unsigned int)inv_step_tiles(hg);
     const unsigned int nf = std::max(1u, std::min(tiles, 2u * (unsigned int)ctx->num_sms));
     return launch_pdl(ctx, "k_inv_fix_pair", k_inv_fix_pair, dim3(nf, 2), dim3(256), 0, p);

@@ -180,6 +180,14 @@ const fw_invert_params kSynInvert = {20, 0.001, 0.1, 1};
 
 }  // namespace
 
+// How many sides one launch of the smoothing and the composition takes: they hand a field on through
+// L2 (126 MB), and two fields that do not fit go one side after the other (193 x 229 x 193, 102 MB a
+// field: 1738 us an iteration with both in one launch, 1718 in turn; 96 x 114 x 96, 13 MB: 357 and
+// 361).
+int syn_sides_together(const HostGrid& g) {
+    return 2 * 12 * plane_stride(g.count()) > (100LL << 20) ? 1 : 2;
+}
+
 // Adds a WHILE node on an existing handle at the capture position of `s`.
 int add_while_node(cudaStream_t s, cudaGraphConditionalHandle handle, cudaGraph_t* body) {
     cudaStreamCaptureStatus status;
@@ -247,14 +255,6 @@ int enqueue_invert_pair(fw_ctx* ctx, bool graph, fw_field* const field[2], fw_fi
 }
 
 unsigned int blocks256(long long n) { return (unsigned int)((n + 255) / 256); }
-
-// How many sides one launch of the smoothing and the composition takes: they hand a field on through
-// L2 (126 MB), and two fields that do not fit go one side after the other (193 x 229 x 193, 102 MB a
-// field: 1738 us an iteration with both in one launch, 1718 in turn; 96 x 114 x 96, 13 MB: 357 and
-// 361).
-int sides_together(const HostGrid& g) {
-    return 2 * 12 * plane_stride(g.count()) > (100LL << 20) ? 1 : 2;
-}
 
 // The kernels of one iteration (syn.rs:890-958) on ctx->stream.
 int enqueue_iteration(fw_ctx* ctx, bool graph, const fw_syn_recipe* r, Level& L,
@@ -342,7 +342,7 @@ int enqueue_iteration(fw_ctx* ctx, bool graph, const fw_syn_recipe* r, Level& L,
     fw_field* field[2] = {L.F, L.M};
     fw_field* inverse[2] = {L.Fi, L.Mi};
     // The composition is in place: every voxel reads its own field value and the update elsewhere.
-    const int sides = sides_together(L.grid);
+    const int sides = syn_sides_together(L.grid);
     for (int s = 0; s < 2; s += sides) {
         if (r->update_field_variance > 0.0) {
             bool in_tmp = false;
@@ -857,7 +857,7 @@ int syn_run_device(fw_ctx* ctx, const fw_syn_recipe* r, const fw_image* const* f
                                                 all[q].inversions[s + 2].iterations});
                 ctx->stats.kernel_launches +=
                     kernels_per_iteration(r, (fixed_mask ? 1 : 0) + (moving_mask ? 1 : 0),
-                                          prior != nullptr, sides_together(g));
+                                          prior != nullptr, syn_sides_together(g));
             }
             if (graphs) ctx->stats.kernel_launches += (uint64_t)graph_levels;
             if (records && cap > 0)

@@ -692,12 +692,12 @@ int fw_batch_syn_run(fw_ctx* ctx, const fw_syn_recipe* recipe, const fw_image* c
 
 /* ---- profiling (crates/fastwarp-gpu/src/profiler.rs:8-60: per-op device timestamps) ----- */
 
-/* Times `reps` launches of each kernel of one SyN iteration on the grid of `fixed` with CUDA
- * events on the context's stream: mean ms per launch and algorithmic bytes per launch of
- * [0] warp, [1] CC pair, [2] Gaussian smoothing + max norm, [3] compose + scale,
- * [4] one inversion body (its bound, step and fix kernels: measurement and update of every
- * voxel), [5] the body's bound kernel alone (the error on one voxel in 64), [6] its fix kernel
- * alone (the update of the tiles the step left for the clamp; bytes counts their voxels). */
+/* Times `reps` runs of each step of one SyN iteration on the grid of `fixed` with CUDA events on
+ * the context's stream, both sides (fixed and moving) by the kernels the iteration launches: mean ms
+ * and algorithmic bytes of [0] the warps, [1] the CC pair, [2] Gaussian smoothing + max norm, [3]
+ * compose + scale, [4] one inversion body (its bound, step and fix kernels: measurement and update
+ * of every voxel), [5] the body's bound kernel alone (the error on one voxel in 64), [6] its fix
+ * kernel alone (the update of the tiles the step left for the clamp; bytes counts their voxels). */
 int fw_time_kernels(fw_ctx* ctx, const fw_image* fixed, const fw_image* moving, int32_t radius,
                     double variance, int32_t reps, double ms[7], double bytes[7]);
 
