@@ -63,7 +63,7 @@ struct MiMap {
     double h[3][3];  // index offset of +half a spacing along physical axis d (central difference)
     DevGrid m;
     int bins;
-    int aligned;     // every h[d] lies along index axis d
+    int aligned;     // every h[d] lies along index axis d, upwards
     double mmin, mmax, mbin, mnmin;
     double isp[3];   // 1 / spacing of the moving image
 };
@@ -394,7 +394,7 @@ __device__ __forceinline__ void mi_finish_body(const unsigned long long* h, int 
 }
 
 // The moving value and the three half-spacing differences v(c + h) - v(c - h) of a sample whose
-// probes move along one index axis each (an axis-aligned image), from 20 voxels: an axis's probes lie
+// probes move up and down one index axis each (MiMap::aligned), from 20 voxels: an axis's probes lie
 // a voxel apart, so their corners are the sample's own eight and, per axis, four more on one side.
 // The sample's eight and the probes' 48 reads came to two thirds of the gradient pass in L1
 // wavefronts (samples four voxels apart in a warp: five lines a load). False where a corner is
@@ -1052,7 +1052,7 @@ MiMap make_map(const fw_mi_level* L, const fw_linear_transform* t) {
     mp.aligned = 1;
     for (int d = 0; d < 3; ++d)
         for (int r = 0; r < 3; ++r)
-            if (r != d && mp.h[d][r] != 0.0) mp.aligned = 0;
+            if (r == d ? !(mp.h[d][r] > 0.0) : mp.h[d][r] != 0.0) mp.aligned = 0;
     for (int d = 0; d < 3; ++d) mp.isp[d] = 1.0 / g.sp[d];
     mp.m = dev_grid(g);
     mp.bins = L->binning.bins;

@@ -164,6 +164,22 @@ def test_dense_histogram_merges_its_words_before_they_overflow(backend):
     assert np.allclose(out[0], out[1], rtol=1e-12, atol=0.0)
 
 
+@pytest.mark.parametrize("direction", [np.diag([-1.0, -1.0, 1.0]), np.diag([1.0, 1.0, -1.0]),
+                                       np.array([[0, 0, 1.0], [1, 0, 0], [0, 1, 0]]),
+                                       np.array([[0, -1.0, 0], [0, 0, -1.0], [1, 0, 0]])])
+def test_gradient_on_flipped_and_permuted_axes_matches(backend, direction):
+    """The orientations of scanners: probes that run down an index axis or along another one."""
+    og, g, f, m, kept, fbin, b = setup((19, 17, 15), (1.0, 2.0, 0.8), (1.0, -2.0, 3.0), direction, seed=8)
+    level = CudaLinearEngine(backend).prepare_level(g, m, kept, fbin, b)
+    kw = transforms(tuple(kept.mean(0)))["euler"]
+    v, d = level.value_and_derivative(linear_transform(**kw))
+    wv, wd, wn, _ = O.mi_evaluate(b, og, m, kept, fbin, O.linear_transform(**kw))
+    assert level.num_valid() == wn
+    # float32 sample offsets and interpolation: about 1e-6 of the difference of two values
+    assert abs(v - wv) <= 1e-5 * abs(wv)
+    assert np.linalg.norm(d - wd) <= 5e-4 * np.linalg.norm(wd)
+
+
 def test_dense_pair_on_an_axis_of_half_a_million_voxels(backend):
     """More rows of 8 than the second dimension of a launch holds: the pair of the same image with its
     long axis along x gives the same histograms, and gradients with x and y exchanged."""
