@@ -23,8 +23,7 @@
 // included (328 with every probe of a face's warp from global memory; unmasked 64 x 217 x 165, where
 // every warp holds a face, 311 us with all probes from global memory, 386 with them at the faces, 139).
 // Measured and dropped: z sums in registers (spills at three CTAs: 521 us), 16 rows a tile with one
-// or two voxels a thread (363-424 us), two CTAs an SM without spills (374 us), thinner z chunks on
-// coarse grids (no change: the call's fixed cost).
+// or two voxels a thread (363-424 us), two CTAs an SM without spills (374 us).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -740,11 +739,11 @@ __global__ void __launch_bounds__(CC_NT, CC_MIN_BLOCKS) k_cc_pair_batch(
 }
 
 // Grid of a launch: TX x TY column tiles times z chunks. About three and a half waves of resident
-// CTAs (measured at the 193 x 229 x 193 finest level, r = 4: 8 chunks 0.398 ms, 5 chunks 0.401 ms,
-// 2 chunks -- less than one wave -- 0.426 ms), with chunks no thinner than 2R slices, the filling
-// steps every chunk pays before its first output -- except where that leaves resident slots empty (the
-// coarse levels), where chunks go down to 4 slices: an iteration at 48 x 57 x 48 takes 116 us with
-// chunks of 8, 110 with 4 or 3, 112 with 2.
+// CTAs (measured at the 193 x 229 x 193 finest level, r = 4: 8 chunks 0.287 ms, 5 chunks 0.303, 12
+// chunks 0.301, 1 chunk 0.426), with chunks no thinner than 2R slices, the filling steps every chunk
+// pays before its first output -- except where that leaves resident slots empty (the coarse levels),
+// where chunks go down to 4 slices: at 48 x 57 x 48 the kernel takes 26 us with 5 chunks, 19 with 12, 17
+// with 16 or 24, and an iteration 116 us with chunks of 8 slices, 110 with 4 or 3, 112 with 2.
 template <int R, int TY, bool MK, int MODE, class Acc = SumF64>
 int plan_launch(CcArgs& a, int num_sms, dim3* grid) {
     using L = Layout<R, TY, MK>;

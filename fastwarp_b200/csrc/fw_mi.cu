@@ -812,7 +812,7 @@ __device__ __forceinline__ void dense_outputs(double w0, double w1, float gm[3],
 // once; any other direction takes the exact probes of every voxel. Bound by the f64 spline weights
 // and the eight ratio reads from shared memory. The pair's whole call at 193 x 229 x 193: 1420 us with
 // a voxel a thread over a 296-block grid (the pass 494) and the histogram of 64-bit cells, 336 with
-// columns in tiles of 32 x 8 (the pass 185), 323 now; turned 2120, 1390 and 960. At 1 x 1000 x 1000, where
+// columns in tiles of 32 x 8 (the pass 185), 323 now (174); turned 2120, 1390 and 960. At 1 x 1000 x 1000, where
 // such a tile has one column in 32: 172, 560 and 107 us.
 template <bool IDENTITY>
 __global__ void __launch_bounds__(MI_THREADS) k_dense_deriv(
